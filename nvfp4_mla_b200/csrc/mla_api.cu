@@ -12,6 +12,7 @@
 #include "mla_decode_sm100.cuh"
 #include "mla_decode_vt_sm100.cuh"
 #include "mla_decode_hm_sm100.cuh"
+#include "mla_decode_hm16_sm100.cuh"
 #include "mla_dequant.cuh"
 #include "mla_quantize.cuh"
 #include "mla_schedule.cuh"
@@ -41,7 +42,8 @@ constexpr int kMaxDevices = 64;
 struct DeviceInfo {
   bool ready = false;
   int sm_count = 0;
-  int hm_pairs = 0;  // CTA pairs (clusters of two) of the heads-as-M kernel that can be resident at once; 0 = do not use it
+  int hm_pairs[2] = {0, 0};  // CTA pairs (clusters of two) of the 16-bit and 8-bit heads-as-M kernels that can be resident at
+                             // once; 0 = do not use it
 };
 std::mutex g_mutex;
 DeviceInfo g_devices[kMaxDevices];
@@ -50,18 +52,31 @@ using DecodeKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtens
 // staging slots of 64 tokens next to the V tile (one FP16 tile of 128 KB, or two E4M3 tiles of 64 KB)
 constexpr int kRawSlots8 = 3;
 constexpr int kRawSlotsHm = 4;  // heads-as-M kernel: staging slots of 32 tokens
-// Heads per CTA (the N of both MMAs). One conversion of a tile serves all of the CTA's heads, so more heads per CTA
-// means less conversion work per head; 32 fit next to the tiles only in the 8-bit mode (tensor memory and shared memory).
-// With 128 heads per request the 8-bit mode runs the heads-as-M kernel: a pair of CTAs per 128 heads (each CTA
-// accumulates half of the output channels), scheduled as one unit, so the schedule sees half as many "CTAs".
+// Heads per CTA or CTA pair. One conversion of a tile serves all of them, so more heads per CTA means less conversion
+// work per head.
+//   8-bit mode : 128 heads run the heads-as-M kernel (a pair of CTAs per 128 heads, each CTA accumulates half of the output
+//                channels; the pair is one unit of the schedule), 32 or 16 heads per CTA the tokens-as-M kernel.
+//   16-bit mode: from kHm16MinHeads heads on, groups of at most 128 (as equal as multiples of 16 allow) run the 16-bit
+//                heads-as-M kernel, fewer the 16-head kernel.
+// The line at 64: 32 requests of 500..16000 tokens with 64 heads take 166 us here against 172 as four groups of 16; a pair
+// takes as long for 48 rows as for 128, the 16-head kernel a quarter less for three groups than for four.
 // `limit` caps the grouping (a caller with little scratch asks for a narrower one: the partial results of a CTA take
 // 2 KB per head).
+constexpr int kHm16MinHeads = 64;
 int heads_per_cta(int heads, int precision, const DeviceInfo& d, int limit = 128) {
-  if (precision != NVFP4_MLA_PRECISION_FP8) return 16;
-  return heads % 128 == 0 && d.hm_pairs > 0 && limit >= 128 ? 128 : heads % 32 == 0 && limit >= 32 ? 32 : 16;
+  if (precision != NVFP4_MLA_PRECISION_FP8) {
+    if (heads < kHm16MinHeads || d.hm_pairs[0] <= 0 || limit < 128) return 16;
+    const int groups = (heads + mla::kH16Rows - 1) / mla::kH16Rows;
+    return ((heads + groups - 1) / groups + 15) / 16 * 16;
+  }
+  return heads % 128 == 0 && d.hm_pairs[1] > 0 && limit >= 128 ? 128 : heads % 32 == 0 && limit >= 32 ? 32 : 16;
 }
-int schedule_units(const DeviceInfo& d, int hpc) { return hpc == 128 ? d.hm_pairs : d.sm_count; }
-int ctas_per_unit(int hpc) { return hpc == 128 ? 2 : 1; }
+bool runs_on_pairs(int hpc) { return hpc > 32; }
+int schedule_units(const DeviceInfo& d, int precision, int hpc) {
+  return runs_on_pairs(hpc) ? d.hm_pairs[precision == NVFP4_MLA_PRECISION_FP8] : d.sm_count;
+}
+int ctas_per_unit(int hpc) { return runs_on_pairs(hpc) ? 2 : 1; }
+// the kernels that take tensor maps (all but the 16-bit heads-as-M kernel)
 DecodeKernel decode_kernel(int precision, int hpc) {
   if (precision == NVFP4_MLA_PRECISION_FP8)
     return hpc == 128  ? mla::mla_decode_hm_kernel<kRawSlotsHm>
@@ -71,15 +86,20 @@ DecodeKernel decode_kernel(int precision, int hpc) {
 }
 unsigned decode_threads(int precision, int hpc) {
   if (precision == NVFP4_MLA_PRECISION_FP8) return hpc == 128 ? mla::kHmThreads : mla::kDecodeThreads;
-  return mla::kVtThreads;
+  return hpc > 16 ? mla::kH16Threads : mla::kVtThreads;
 }
 size_t decode_smem(int precision, int hpc) {
   if (precision == NVFP4_MLA_PRECISION_FP8)
     return hpc == 128  ? mla::hm_smem_bytes<kRawSlotsHm>()
            : hpc == 32 ? mla::decode_smem_bytes<32, kRawSlots8, true>()
                        : mla::decode_smem_bytes<16, kRawSlots8, true>();
-  return mla::vt_smem_bytes();
+  return hpc > 16 ? mla::h16_smem_bytes() : mla::vt_smem_bytes();
 }
+const void* decode_entry(int precision, int hpc) {
+  if (precision != NVFP4_MLA_PRECISION_FP8 && hpc > 16) return reinterpret_cast<const void*>(mla::mla_decode_hm16_kernel);
+  return reinterpret_cast<const void*>(decode_kernel(precision, hpc));
+}
+static_assert(mla::h16_smem_bytes() <= 232448, "16-bit heads-as-M kernel exceeds the shared memory a CTA can opt in to");
 static_assert(mla::hm_smem_bytes<kRawSlotsHm>() <= 232448, "heads-as-M kernel exceeds the shared memory a CTA can opt in to");
 static_assert(mla::decode_smem_bytes<32, kRawSlots8, true>() <= 232448 && mla::decode_smem_bytes<16, kRawSlots8, true>() <= 232448 &&
                   mla::vt_smem_bytes() <= 232448,
@@ -99,24 +119,27 @@ int device_info(DeviceInfo** out) {
     MLA_CUDA(cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev));
     for (int prec : {NVFP4_MLA_PRECISION_BF16, NVFP4_MLA_PRECISION_FP8})
       for (int hpc : {16, 32, 128})
-        MLA_CUDA(cudaFuncSetAttribute(decode_kernel(prec, hpc), cudaFuncAttributeMaxDynamicSharedMemorySize,
+        MLA_CUDA(cudaFuncSetAttribute(decode_entry(prec, hpc), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       int(decode_smem(prec, hpc))));
-    {  // clusters of two need both SMs in one GPC: ask how many can be resident rather than assuming sm_count / 2
+    for (int prec : {NVFP4_MLA_PRECISION_BF16, NVFP4_MLA_PRECISION_FP8}) {
+      // clusters of two need both SMs in one GPC: ask how many can be resident rather than assuming sm_count / 2
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(unsigned(d.sm_count / 2 * 2)), cfg.blockDim = dim3(mla::kHmThreads);
-      cfg.dynamicSmemBytes = decode_smem(NVFP4_MLA_PRECISION_FP8, 128);
+      cfg.gridDim = dim3(unsigned(d.sm_count / 2 * 2)), cfg.blockDim = dim3(decode_threads(prec, 128));
+      cfg.dynamicSmemBytes = decode_smem(prec, 128);
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
       cfg.attrs = attr, cfg.numAttrs = 1;
       int clusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&clusters, decode_kernel(NVFP4_MLA_PRECISION_FP8, 128), &cfg) != cudaSuccess) {
+      if (cudaOccupancyMaxActiveClusters(&clusters, decode_entry(prec, 128), &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
         clusters = 0;
       }
-      d.hm_pairs = clusters < d.sm_count / 2 ? clusters : d.sm_count / 2;
+      int& pairs = d.hm_pairs[prec == NVFP4_MLA_PRECISION_FP8];
+      pairs = clusters < d.sm_count / 2 ? clusters : d.sm_count / 2;
       if (getenv("NVFP4_MLA_DEBUG"))
-        fprintf(stderr, "nvfp4_mla_b200: device %d: %d SMs, %d resident CTA pairs for the 128-head kernel\n", dev, d.sm_count, d.hm_pairs);
+        fprintf(stderr, "nvfp4_mla_b200: device %d: %d SMs, %d resident CTA pairs for the %s heads-as-M kernel\n", dev, d.sm_count, pairs,
+                prec == NVFP4_MLA_PRECISION_FP8 ? "8-bit" : "16-bit");
     }
     d.ready = true;
   }
@@ -201,7 +224,7 @@ int problem_of(int batch, int heads, int max_kv_len, int num_splits, int n_cta, 
   const int splits = num_splits > 0 ? num_splits : 1;
   const long long len = max_kv_len > 1 ? max_kv_len : 1;
   const long long chunk = ((len + splits - 1) / splits + mla::TILE - 1) / mla::TILE * mla::TILE;
-  pb->batch = batch, pb->heads = heads, pb->heads_per_cta = hpc, pb->head_groups = heads / hpc;
+  pb->batch = batch, pb->heads = heads, pb->heads_per_cta = hpc, pb->head_groups = (heads + hpc - 1) / hpc;
   pb->splits = splits, pb->chunk = int(chunk), pb->n_cta = n_cta;
   MLA_CHECK((long long)batch * splits <= mla::kSchedMaxBZ, "batch * num_splits = %lld exceeds %d", (long long)batch * splits,
             mla::kSchedMaxBZ);
@@ -231,7 +254,7 @@ static int64_t workspace_bytes_of(int batch, int heads, int num_splits, int prec
   if (device_info(&d)) return -1;
   mla::Problem pb;
   const int hpc = heads_per_cta(heads, precision, *d, hpc_limit);
-  if (problem_of(batch, heads, 1, num_splits, schedule_units(*d, hpc), hpc, &pb)) return -1;
+  if (problem_of(batch, heads, 1, num_splits, schedule_units(*d, precision, hpc), hpc, &pb)) return -1;
   return int64_t(mla::ws_layout(pb.n_cta, pb.items(), pb.heads_per_cta).total);
 }
 
@@ -245,7 +268,7 @@ int nvfp4_mla_decode_launches(int batch, int heads, int max_kv_len, int num_spli
   if (device_info(&d)) return -1;
   mla::Problem pb;
   const int hpc = heads_per_cta(heads, precision, *d, 128);
-  if (problem_of(batch, heads, max_kv_len, num_splits, schedule_units(*d, hpc), hpc, &pb)) return -1;
+  if (problem_of(batch, heads, max_kv_len, num_splits, schedule_units(*d, precision, hpc), hpc, &pb)) return -1;
   if (batch == 0) return 0;
   return schedules_itself(pb, precision, hpc) ? 2 : 3;
 }
@@ -279,17 +302,18 @@ static int decode_impl(const void* q_nope, const void* q_pe, const uint8_t* ckv_
   if (device_info(&d)) return 1;
   mla::Problem pb;
   const int hpc = heads_per_cta(heads, precision, *d, hpc_limit);
-  if (problem_of(batch, heads, max_kv_len, num_splits, schedule_units(*d, hpc), hpc, &pb)) return 1;
+  if (problem_of(batch, heads, max_kv_len, num_splits, schedule_units(*d, precision, hpc), hpc, &pb)) return 1;
   if (batch == 0) return 0;
   const mla::WsLayout L = mla::ws_layout(pb.n_cta, pb.items(), pb.heads_per_cta);
   MLA_CHECK(workspace_bytes >= int64_t(L.total), "workspace too small: %lld bytes given, %lld needed", (long long)workspace_bytes,
             (long long)L.total);
 
+  const bool hm16 = precision != NVFP4_MLA_PRECISION_FP8 && hpc > 16;  // loads with plain instructions: no tensor maps
   CUtensorMap ckv_map, sf_map, kpe_map;
   const int slot_rows = hpc == 128 ? mla::kHmRows : mla::HALF;  // tokens per staging slot of the kernel that will run
-  if (make_row_map(ckv_cache, num_pages * page_size, 256, 128, page_size, slot_rows, CU_TENSOR_MAP_SWIZZLE_128B, &ckv_map)) return 1;
-  if (make_row_map(ckv_sf_cache, num_pages * page_size, 32, 32, page_size, slot_rows, CU_TENSOR_MAP_SWIZZLE_32B, &sf_map)) return 1;
-  if (make_row_map(kpe_cache, num_pages * page_size, 64, 64, page_size, slot_rows, CU_TENSOR_MAP_SWIZZLE_64B, &kpe_map)) return 1;
+  if (!hm16 && make_row_map(ckv_cache, num_pages * page_size, 256, 128, page_size, slot_rows, CU_TENSOR_MAP_SWIZZLE_128B, &ckv_map)) return 1;
+  if (!hm16 && make_row_map(ckv_sf_cache, num_pages * page_size, 32, 32, page_size, slot_rows, CU_TENSOR_MAP_SWIZZLE_32B, &sf_map)) return 1;
+  if (!hm16 && make_row_map(kpe_cache, num_pages * page_size, 64, 64, page_size, slot_rows, CU_TENSOR_MAP_SWIZZLE_64B, &kpe_map)) return 1;
 
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   int* header = reinterpret_cast<int*>(ws + L.header);
@@ -319,9 +343,12 @@ static int decode_impl(const void* q_nope, const void* q_pe, const uint8_t* ckv_
   P.cta_range_out = cta_range, P.segs_out = segs;
   Profile* prof = g_profile && g_profile->used < int(g_profile->start.size()) ? g_profile : nullptr;
   if (prof) MLA_CUDA(cudaEventRecord(prof->start[prof->used], st));
-  MLA_CUDA(launch_dependent_cluster(decode_kernel(precision, hpc), dim3(pb.n_cta * ctas_per_unit(hpc)),
-                                    dim3(decode_threads(precision, hpc)), decode_smem(precision, hpc), st,
-                                    unsigned(ctas_per_unit(hpc)), ckv_map, sf_map, kpe_map, P));
+  const dim3 grid(pb.n_cta * ctas_per_unit(hpc)), block(decode_threads(precision, hpc));
+  if (hm16)
+    MLA_CUDA(launch_dependent_cluster(mla::mla_decode_hm16_kernel, grid, block, decode_smem(precision, hpc), st, 2u, P));
+  else
+    MLA_CUDA(launch_dependent_cluster(decode_kernel(precision, hpc), grid, block, decode_smem(precision, hpc), st,
+                                      unsigned(ctas_per_unit(hpc)), ckv_map, sf_map, kpe_map, P));
   if (prof) MLA_CUDA(cudaEventRecord(prof->stop[prof->used++], st));
 
   // few rows: four thread groups share a row's partials; many rows: one group per row keeps the CTAs small

@@ -1,0 +1,91 @@
+"""The 16-bit heads-as-M kernel (64 heads and more) against the numpy oracle, where it can go wrong: the smallest and the
+unequal head groups, quadrants without live rows, lengths around its 64-token tile and its 32-token share per CTA, every
+kind of page, many short requests per CTA pair, and the sign of the softmax scale.
+Tolerances as in test_decode_gpu.py: max-abs <= 2e-2, rel-L2 < 4e-3, natural-log LSE <= 1e-3."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+import mla_oracle as O
+import nvfp4_mla_b200 as mla
+from nvfp4_mla_b200.testing import SM_SCALE, SyntheticCache
+from util import oracle_reference
+
+pytestmark = pytest.mark.gpu
+LN2 = math.log(2.0)
+
+
+def run(c, sm_scale=SM_SCALE, num_splits=0):
+    args = (c.q_nope, c.q_pe, c.ckv_cache, c.ckv_sf_cache, c.kpe_cache, c.page_table, c.kv_lens, sm_scale, c.ckv_scale, c.kpe_scale)
+    longest = max(c.kv_lens_list)
+    out = mla.decode(*args, max_kv_len=longest, num_splits=num_splits)
+    _, lse2 = mla.decode_partial(*args, max_kv_len=longest, num_splits=num_splits)
+    assert mla.workspace_status() == 0
+    return out.float().cpu().numpy(), lse2.cpu().numpy() * LN2
+
+
+def check(c, sm_scale=SM_SCALE, num_splits=0):
+    got, lse = run(c, sm_scale, num_splits)
+    want, want_lse = oracle_reference(c, sm_scale)
+    live = [b for b, n in enumerate(c.kv_lens_list) if n > 0]
+    assert np.abs(got - want).max() <= 2e-2
+    assert O.rel_l2(got[live], want[live]) < 4e-3
+    assert np.abs(lse[live] - want_lse[live]).max() <= 1e-3
+    for b, n in enumerate(c.kv_lens_list):
+        if n == 0:
+            assert (got[b] == 0).all() and np.isneginf(lse[b]).all()
+
+
+@pytest.mark.parametrize("heads", [64, 80, 112, 128, 144, 192, 256])
+@pytest.mark.parametrize("num_splits", [0, 3])
+def test_head_groups(heads, num_splits):
+    check(SyntheticCache([513, 64, 1], 64, heads, None, None, seed=heads).to("cuda"), num_splits=num_splits)
+
+
+@pytest.mark.parametrize("page_size", [1, 2, 8, 16, 32, 64, 256])
+def test_lengths_around_the_tile(page_size):
+    lens = [1, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 0, 191, 192, 193, 257]
+    check(SyntheticCache(lens, page_size, 64, 0.5, 2.0, seed=page_size).to("cuda"))
+
+
+def test_many_short_requests_per_pair():
+    rng = np.random.default_rng(3)
+    check(SyntheticCache([int(x) for x in rng.integers(1, 200, 300)], 16, 80, None, None, seed=5).to("cuda"))
+
+
+@pytest.mark.parametrize("sm_scale", [-SM_SCALE, 0.0])
+def test_sign_of_the_softmax_scale(sm_scale):
+    check(SyntheticCache([300, 65], 64, 128, 0.5, 2.0, seed=9).to("cuda"), sm_scale)
+
+
+def test_wide_range_of_query_magnitudes_and_non_finite_elements():
+    c = SyntheticCache([500, 129], 64, 64, 0.01, 0.01, seed=2).to("cuda")
+    c.q_nope[:, :, 7] *= 64.0                       # outlier channel
+    c.q_nope[:, 3] *= 2.0 ** -60                    # a tiny row
+    c.q_pe[:, 5] *= 32.0                            # the rope part decides the row's scale
+    check(c)
+    clean, _ = run(c)
+    c.q_nope[0, 1, 11], c.q_nope[0, 2, 300], c.q_pe[1, 4, 3] = float("nan"), float("inf"), -float("inf")
+    got, _ = run(c)
+    assert np.isfinite(got).all()  # a non-finite element counts as 0
+    hit = [(0, 1), (0, 2), (1, 4)]
+    for b in range(2):
+        for h in range(64):
+            if (b, h) not in hit:
+                assert np.array_equal(got[b, h], clean[b, h])
+    c.q_nope[0, 1, 11], c.q_nope[0, 2, 300], c.q_pe[1, 4, 3] = 0.0, 0.0, 0.0
+    zeroed, _ = run(c)
+    assert np.array_equal(got, zeroed)
+
+
+@pytest.mark.parametrize("page_size", [16, 64])
+def test_page_ids_are_range_checked(page_size):
+    c = SyntheticCache([200, 90], page_size, 128, None, None, seed=4).to("cuda")
+    good, _ = run(c)
+    c.page_table[1, 0] = c.ckv_cache.shape[0] + 5
+    args = (c.q_nope, c.q_pe, c.ckv_cache, c.ckv_sf_cache, c.kpe_cache, c.page_table, c.kv_lens, SM_SCALE, c.ckv_scale, c.kpe_scale)
+    out = mla.decode(*args, max_kv_len=200)
+    assert mla.workspace_status(clear=True) == 3
+    assert np.array_equal(out[0].float().cpu().numpy(), good[0]) and torch.isfinite(out.float()).all()
