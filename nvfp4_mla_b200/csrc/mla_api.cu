@@ -1,5 +1,6 @@
 // C ABI of libnvfp4_mla_b200.so: argument validation, the TMA descriptor of the cache, and kernel launches.
 // Declarations and their documentation: include/nvfp4_mla_b200.h.
+#include <climits>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -42,8 +43,7 @@ constexpr int kMaxDevices = 64;
 struct DeviceInfo {
   bool ready = false;
   int sm_count = 0;
-  int hm_pairs[2] = {0, 0};  // CTA pairs (clusters of two) of the 16-bit and 8-bit heads-as-M kernels that can be resident at
-                             // once; 0 = do not use it
+  int hm_pairs = 0;  // CTA pairs (clusters of two) of the 8-bit heads-as-M kernel that can be resident at once; 0 = do not use it
 };
 std::mutex g_mutex;
 DeviceInfo g_devices[kMaxDevices];
@@ -56,24 +56,32 @@ constexpr int kRawSlotsHm = 4;  // heads-as-M kernel: staging slots of 32 tokens
 // work per head.
 //   8-bit mode : 128 heads run the heads-as-M kernel (a pair of CTAs per 128 heads, each CTA accumulates half of the output
 //                channels; the pair is one unit of the schedule), 32 or 16 heads per CTA the tokens-as-M kernel.
-//   16-bit mode: from kHm16MinHeads heads on, groups of at most 128 (as equal as multiples of 16 allow) run the 16-bit
-//                heads-as-M kernel, fewer the 16-head kernel.
-// The line at 64: 32 requests of 500..16000 tokens with 64 heads take 166 us here against 172 as four groups of 16; a pair
-// takes as long for 48 rows as for 128, the 16-head kernel a quarter less for three groups than for four.
+//   16-bit mode: groups of at most 128 heads (as equal as multiples of 16 allow) run the 16-bit heads-as-M kernel where it is
+//                the faster one (below), otherwise 16 heads per CTA the 16-head kernel.
 // `limit` caps the grouping (a caller with little scratch asks for a narrower one: the partial results of a CTA take
 // 2 KB per head).
+//
+// The 16-bit heads-as-M kernel against the 16-head kernel, us a call: a pair of CTAs takes as long for 48 rows as for 128, so
+// it needs enough heads, and its query load and pipeline are longer, so it needs more than about four 128-token tiles x 16
+// heads per SM: (heads, batch, length) 64,1,1K: 31 against 24 us a call; 128,1,8K: 35 / 33; 64,32,512: 31 / 32; 128,32,512:
+// 40 / 54; 64,128,300: 64 / 76; 64,32 ragged 500..16K: 137 / 171; 128,64,16K: 415 / 833; 128,2,1M: 884 / 1740.
 constexpr int kHm16MinHeads = 64;
-int heads_per_cta(int heads, int precision, const DeviceInfo& d, int limit = 128) {
-  if (precision != NVFP4_MLA_PRECISION_FP8) {
-    if (heads < kHm16MinHeads || d.hm_pairs[0] <= 0 || limit < 128) return 16;
-    const int groups = (heads + mla::kH16Rows - 1) / mla::kH16Rows;
-    return ((heads + groups - 1) / groups + 15) / 16 * 16;
-  }
-  return heads % 128 == 0 && d.hm_pairs[1] > 0 && limit >= 128 ? 128 : heads % 32 == 0 && limit >= 32 ? 32 : 16;
+bool wants_hm16(int heads, int batch, int max_kv_len, const DeviceInfo& d) {
+  const long long tiles = (long long)batch * ((max_kv_len + mla::TILE - 1) / mla::TILE) * (heads / 16);
+  return heads >= kHm16MinHeads && tiles > 4ll * d.sm_count;
+}
+int hm16_group(int heads) {
+  const int groups = (heads + mla::kH16Rows - 1) / mla::kH16Rows;
+  return ((heads + groups - 1) / groups + 15) / 16 * 16;
+}
+int heads_per_cta(int heads, int precision, const DeviceInfo& d, int limit, int batch, int max_kv_len) {
+  if (precision != NVFP4_MLA_PRECISION_FP8) return limit >= 128 && wants_hm16(heads, batch, max_kv_len, d) ? hm16_group(heads) : 16;
+  return heads % 128 == 0 && d.hm_pairs > 0 && limit >= 128 ? 128 : heads % 32 == 0 && limit >= 32 ? 32 : 16;
 }
 bool runs_on_pairs(int hpc) { return hpc > 32; }
 int schedule_units(const DeviceInfo& d, int precision, int hpc) {
-  return runs_on_pairs(hpc) ? d.hm_pairs[precision == NVFP4_MLA_PRECISION_FP8] : d.sm_count;
+  if (!runs_on_pairs(hpc)) return d.sm_count;
+  return precision == NVFP4_MLA_PRECISION_FP8 ? d.hm_pairs : d.sm_count / 2;  // (the 16-bit pairs are not clusters)
 }
 int ctas_per_unit(int hpc) { return runs_on_pairs(hpc) ? 2 : 1; }
 // the kernels that take tensor maps (all but the 16-bit heads-as-M kernel)
@@ -121,25 +129,22 @@ int device_info(DeviceInfo** out) {
       for (int hpc : {16, 32, 128})
         MLA_CUDA(cudaFuncSetAttribute(decode_entry(prec, hpc), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       int(decode_smem(prec, hpc))));
-    for (int prec : {NVFP4_MLA_PRECISION_BF16, NVFP4_MLA_PRECISION_FP8}) {
-      // clusters of two need both SMs in one GPC: ask how many can be resident rather than assuming sm_count / 2
+    {  // clusters of two need both SMs in one GPC: ask how many can be resident rather than assuming sm_count / 2
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(unsigned(d.sm_count / 2 * 2)), cfg.blockDim = dim3(decode_threads(prec, 128));
-      cfg.dynamicSmemBytes = decode_smem(prec, 128);
+      cfg.gridDim = dim3(unsigned(d.sm_count / 2 * 2)), cfg.blockDim = dim3(mla::kHmThreads);
+      cfg.dynamicSmemBytes = decode_smem(NVFP4_MLA_PRECISION_FP8, 128);
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
       cfg.attrs = attr, cfg.numAttrs = 1;
       int clusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&clusters, decode_entry(prec, 128), &cfg) != cudaSuccess) {
+      if (cudaOccupancyMaxActiveClusters(&clusters, decode_kernel(NVFP4_MLA_PRECISION_FP8, 128), &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
         clusters = 0;
       }
-      int& pairs = d.hm_pairs[prec == NVFP4_MLA_PRECISION_FP8];
-      pairs = clusters < d.sm_count / 2 ? clusters : d.sm_count / 2;
+      d.hm_pairs = clusters < d.sm_count / 2 ? clusters : d.sm_count / 2;
       if (getenv("NVFP4_MLA_DEBUG"))
-        fprintf(stderr, "nvfp4_mla_b200: device %d: %d SMs, %d resident CTA pairs for the %s heads-as-M kernel\n", dev, d.sm_count, pairs,
-                prec == NVFP4_MLA_PRECISION_FP8 ? "8-bit" : "16-bit");
+        fprintf(stderr, "nvfp4_mla_b200: device %d: %d SMs, %d resident CTA pairs for the 128-head kernel\n", dev, d.sm_count, d.hm_pairs);
     }
     d.ready = true;
   }
@@ -248,14 +253,20 @@ static bool schedules_itself(const mla::Problem& pb, int precision, int hpc) {
          bz * ((pb.chunk + mla::TILE - 1) / mla::TILE + 1) * pb.head_groups < (1ll << 31);
 }
 
-// workspace of one precision mode (the modes may group the heads differently); negative on error
+// Workspace of one precision mode (the modes may group the heads differently); negative on error. In the 16-bit mode the
+// grouping depends on the call's max_kv_len: the size covers either one that `hpc_limit` allows.
 static int64_t workspace_bytes_of(int batch, int heads, int num_splits, int precision, int hpc_limit = 128) {
   DeviceInfo* d;
   if (device_info(&d)) return -1;
-  mla::Problem pb;
-  const int hpc = heads_per_cta(heads, precision, *d, hpc_limit);
-  if (problem_of(batch, heads, 1, num_splits, schedule_units(*d, precision, hpc), hpc, &pb)) return -1;
-  return int64_t(mla::ws_layout(pb.n_cta, pb.items(), pb.heads_per_cta).total);
+  int64_t worst = -1;
+  for (const int max_kv_len : {1, INT_MAX - mla::TILE}) {
+    mla::Problem pb;
+    const int hpc = heads_per_cta(heads, precision, *d, hpc_limit, batch, max_kv_len);
+    if (problem_of(batch, heads, 1, num_splits, schedule_units(*d, precision, hpc), hpc, &pb)) return -1;
+    const int64_t bytes = int64_t(mla::ws_layout(pb.n_cta, pb.items(), pb.heads_per_cta).total);
+    worst = bytes > worst ? bytes : worst;
+  }
+  return worst;
 }
 
 int nvfp4_mla_decode_launches(int batch, int heads, int max_kv_len, int num_splits, int precision) {
@@ -267,7 +278,7 @@ int nvfp4_mla_decode_launches(int batch, int heads, int max_kv_len, int num_spli
   DeviceInfo* d;
   if (device_info(&d)) return -1;
   mla::Problem pb;
-  const int hpc = heads_per_cta(heads, precision, *d, 128);
+  const int hpc = heads_per_cta(heads, precision, *d, 128, batch, max_kv_len);
   if (problem_of(batch, heads, max_kv_len, num_splits, schedule_units(*d, precision, hpc), hpc, &pb)) return -1;
   if (batch == 0) return 0;
   return schedules_itself(pb, precision, hpc) ? 2 : 3;
@@ -301,7 +312,7 @@ static int decode_impl(const void* q_nope, const void* q_pe, const uint8_t* ckv_
   DeviceInfo* d;
   if (device_info(&d)) return 1;
   mla::Problem pb;
-  const int hpc = heads_per_cta(heads, precision, *d, hpc_limit);
+  const int hpc = heads_per_cta(heads, precision, *d, hpc_limit, batch, max_kv_len);
   if (problem_of(batch, heads, max_kv_len, num_splits, schedule_units(*d, precision, hpc), hpc, &pb)) return 1;
   if (batch == 0) return 0;
   const mla::WsLayout L = mla::ws_layout(pb.n_cta, pb.items(), pb.heads_per_cta);
@@ -345,7 +356,7 @@ static int decode_impl(const void* q_nope, const void* q_pe, const uint8_t* ckv_
   if (prof) MLA_CUDA(cudaEventRecord(prof->start[prof->used], st));
   const dim3 grid(pb.n_cta * ctas_per_unit(hpc)), block(decode_threads(precision, hpc));
   if (hm16)
-    MLA_CUDA(launch_dependent_cluster(mla::mla_decode_hm16_kernel, grid, block, decode_smem(precision, hpc), st, 2u, P));
+    MLA_CUDA(launch_dependent(mla::mla_decode_hm16_kernel, grid, block, decode_smem(precision, hpc), st, P));
   else
     MLA_CUDA(launch_dependent_cluster(decode_kernel(precision, hpc), grid, block, decode_smem(precision, hpc), st,
                                       unsigned(ctas_per_unit(hpc)), ckv_map, sf_map, kpe_map, P));

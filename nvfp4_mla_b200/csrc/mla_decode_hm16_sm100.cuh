@@ -10,43 +10,42 @@
 // Both K and V are exact in FP16 (e2m1 x e4m3 has six significant bits), Q is exact after a power-of-two scaling of the
 // row (a BF16 has eight), the accumulators are fp32.
 //
-// O for 128 rows x 512 channels would need all 512 tensor-memory columns, so a PAIR of CTAs (a cluster of two) shares a
-// request: both compute the full scores, CTA `cg` accumulates channels [256 cg, 256 cg + 256). CTA `cg` dequantises
-// tokens [32 cg, 32 cg + 32) of every 64-token tile into its own tile and sends the same bytes to its peer's tile with
-// bulk copies through distributed shared memory. The pair is one unit of the schedule and writes one partial slot.
+// O for 128 rows x 512 channels would need all 512 tensor-memory columns, so a PAIR of CTAs shares a request: both compute
+// the full scores, CTA `cg` accumulates channels [256 cg, 256 cg + 256). The pair is one unit of the schedule and writes one
+// partial slot; its CTAs do not communicate (the second read of a token is an L2 hit). An earlier form was a cluster of two
+// that shared the conversion, each CTA sending half of every tile to its peer by bulk copies through distributed shared
+// memory: 981 us instead of 884 (128 heads, two requests of 1M tokens; 1740 with the 16-head kernel), because a tile's first
+// MMA waited for the peer's PV of two tiles before, its conversion and the transfer.
 //
 // What bounds it from below is the tensor pipe. Per 64-token tile and CTA 20 MMAs of 32 cycles (A in tensor memory), 16 of
-// 48 (A in shared memory, bound by the operand read) and 4 of 128 for PV: 1920 cycles. Storage allows two K/V tiles only
-// (Q 144 KB, O 128 KB and S / P 48 KB of tensor memory + shared memory leave room for 2.2), so a tile is handed over in two
-// parts: A = the nine panels minus this CTA's PV half (free as soon as QK^T has read them), B = the four panels PV reads.
-// The next tile's part A is converted and multiplied while PV of the previous tile still holds part B.
-//
-// Measured, 128 heads, two requests of 1M tokens: 981 us a call against 1725 with the 16-head kernel (eight groups).
+// 48 (A in shared memory, bound by the operand read) and 4 of 128 for PV: 1920 cycles, of about 2700 measured. Storage
+// allows two K/V tiles only (Q 144 KB, O 128 KB and S / P 48 KB of tensor memory + shared memory leave room for 2.2), so a
+// tile is handed over in two parts: A = the nine panels minus this CTA's PV half (free as soon as QK^T has read them), B =
+// the four panels PV reads. The next tile's part A is converted and multiplied while PV of the previous tile still holds
+// part B. What limits a tile now is the softmax warps' serial chain (scores -> vote -> exponentials -> P), behind which S has
+// one buffer only; long calls run at the power limit (about 1.4 GHz).
 //
 // Tensor memory (512 columns): Q latent 0..255: 0..127 | Q rope: 128..159 | S: 160..223 | P: 224..255 | O: 256..511.
-// Warp roles (640 threads): 0-7 softmax + query load + epilogue, 8-15 dequantise (warp = 64-channel panel), 16 QK^T
-// issue, 17 L2 prefetch (at the end it also waits for the peer's last buffer releases, so that no CTA leaves while its
-// peer may still signal it), 18 PV issue. Every wait is bounded (ptx::mbar_wait).
+// Warp roles (896 threads): 0-7 softmax + query load + epilogue, 8-23 dequantise (warp = 32 rows of a 64-channel panel), 24
+// QK^T issue, 25 L2 prefetch, 26 PV issue. Every wait is bounded (ptx::mbar_wait).
 #pragma once
 #include "mla_decode_sm100.cuh"
 
 namespace mla {
 
-constexpr int kH16Threads = 640;
+constexpr int kH16Threads = 896;
 constexpr int kH16Rows = 128;              // query rows per CTA pair = MMA M (at most; the rest of M is dead)
 constexpr int kH16Tile = 64;               // tokens per tile
-constexpr int kH16Own = kH16Tile / 2;      // token rows one CTA of the pair loads and converts per tile
+constexpr int kH16Own = kH16Tile / 2;      // token rows of a tile that one CTA of the pair prefetches into L2
 constexpr int kH16Panel = kH16Tile * 128;  // one 64-channel panel of the FP16 tile
 constexpr int kH16Ahead = 6;               // tiles between a load and its L2 prefetch
-constexpr uint32_t kH16PeerA = 4 * 4096 + 8 * 512, kH16PeerB = 4 * 4096;  // bytes the peer sends per tile, parts A and B
 
 struct H16Smem {
   alignas(1024) uint8_t q[4][kH16Rows * 128];   // latent channels 256..511 of Q, FP16, row = query row, four panels of 64 channels
   alignas(1024) uint8_t kv[2][9][kH16Panel];    // panels 0..7: latent channels, panel 8: rope
   Seg segs[kSegBatch];
-  alignas(8) uint64_t full_a[2], full_b[2];     // part of the tile in place: local convert warps + the peer's bytes
-  // buffer part released, by CTA x of the pair (each CTA keeps the releases of both): part A by its QK^T, part B by its PV
-  uint64_t free_a[2][2], free_b[2][2];          // [x][buffer]
+  alignas(8) uint64_t full_a[2], full_b[2];     // part of the tile in place (eight convert warps each)
+  uint64_t free_a[2], free_b[2];                // buffer part released: part A by QK^T, part B by PV
   uint64_t s_full, s_free;                      // one phase per tile
   uint64_t p_full, pv_done;                     // one phase per tile
   uint64_t q_full;                              // query of the segment in place (8 softmax warps)
@@ -88,9 +87,13 @@ __device__ __forceinline__ void h16_prefetch_rows(const DecodeParams& P, const S
   if (uint32_t(page) >= uint32_t(P.num_pages)) return;
   const int in_page = tok & ((1 << P.page_shift) - 1);
   const long long row = ((long long)page << P.page_shift) + in_page;
-  ptx::prefetch_l2(P.ckv + row * 256), ptx::prefetch_l2(P.ckv + row * 256 + 128);
-  if ((lane & 1) == 0 || in_page == 0) ptx::prefetch_l2(P.kpe + row * 64);
-  if ((lane & 3) == 0 || in_page == 0) ptx::prefetch_l2(P.sf + row * 32);
+  // one request per run of contiguous rows (a page, or this CTA's share of the tile), by the lane of its first row
+  const int run = P.page_shift >= 5 ? kH16Own : 1 << P.page_shift;
+  if ((lane & (run - 1)) == 0) {
+    ptx::bulk_prefetch_l2(P.ckv + row * 256, run * 256);
+    ptx::bulk_prefetch_l2(P.kpe + row * 64, run * 64);
+    ptx::bulk_prefetch_l2(P.sf + row * 32, run * 32);
+  }
 }
 __device__ __forceinline__ void h16_prefetch_role(H16Smem& s, const DecodeParams& P, int n_segs, uint32_t& it, int cg) {
   const int lane = ptx::lane_id();
@@ -122,117 +125,104 @@ __device__ __forceinline__ void h16_prefetch_role(H16Smem& s, const DecodeParams
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// role: dequantise (8 warps) this CTA's 32 token rows of every tile, into its own tile and the peer's. Warp w: panel w
-// (64 channels); a lane takes half a panel row (16 packed bytes = two scale blocks) of rows lane / 2 and 16 + lane / 2,
-// so that a warp's load touches 16 lines and its 16-byte stores are conflict-free. Rope: rows 4 w .. 4 w + 3, eight lanes
-// per row. Rows past the request's end (and rows of a bad page id) are never loaded: zero bytes, zero scale.
-// The loads of tile t + 1 and the page ids of tile t + 2 are in flight while tile t is converted.
+// role: dequantise (16 warps). Warp cw: panel cw % 8 (64 channels), rows [32 (cw / 8), +32) of the tile; a lane takes half a
+// panel row (16 packed bytes = two scale blocks) of rows lane / 2 and 16 + lane / 2, so that a warp's load touches 16 lines
+// and its 16-byte stores are conflict-free. The warps of part A also move the rope panel (8 rows each, eight lanes per row).
+// The cache row of a token is looked up by one lane and handed round by shuffle. Rows past the request's end and rows of a
+// bad page id are never loaded: zero bytes, zero scale. The loads of tile t + 1 are issued as soon as tile t's bytes have
+// been converted, the page ids of tile t + 2 behind them.
 // ---------------------------------------------------------------------------------------------------------------
-struct H16Raw {
-  uint4 w[2];
-  uint32_t sf[2];
-  uint2 rope;
-};
-__device__ __forceinline__ void h16_convert_role(H16Smem& s, const DecodeParams& P, int n_segs, uint32_t& it, int cg) {
+template <bool part_a>  // whether the warp's panel belongs to part A
+__device__ __forceinline__ void h16_convert_warps(H16Smem& s, const DecodeParams& P, int n_segs, uint32_t& it) {
   const int lane = ptx::lane_id();
-  const int w = (threadIdx.x >> 5) - 8, hf = w >> 2, hh = lane & 1;
-  const int r[3] = {lane >> 1, 16 + (lane >> 1), 4 * w + (lane >> 3)};  // two latent rows, one rope row
-  const int ps_mask = (1 << P.page_shift) - 1;
-  const uint32_t peer = uint32_t(cg ^ 1);
+  const int cw = (threadIdx.x >> 5) - 8, w = cw & 7, v = cw >> 3, hh = lane & 1;
+  uint64_t* const full = part_a ? s.full_a : s.full_b;
+  uint64_t* const freed = part_a ? s.free_a : s.free_b;
+  const int rope_row = 8 * (w & 3) + (lane >> 3);  // of this warp's 32 rows; the lane's second one is 4 rows further
+  // per-lane byte offsets: latent chunk c of a row r is at 16 ((4 hh + c) ^ (r % 8)), and r % 8 is the same for both rows
+  const uint32_t kv0 = ptx::smem_u32(s.kv[0][0]);
+  const uint32_t dst0 = kv0 + w * kH16Panel + (32 * v + (lane >> 1)) * 128 + ((uint32_t(4 * hh) ^ uint32_t((lane >> 1) & 4)) << 4);
+  const uint32_t swz = uint32_t((lane >> 1) & 3) << 4;
+  const uint32_t rope0 = kv0 + 8 * kH16Panel + (32 * v + rope_row) * 128, rope_c = uint32_t(lane & 7), rope_s = uint32_t(rope_row & 7);
+  const uint8_t* const ckv0 = P.ckv + 32 * w + 16 * hh;
+  const uint8_t* const sf0 = P.sf + 4 * w + 2 * hh;
+  const uint8_t* const kpe0 = P.kpe + 8 * (lane & 7);
   for (int si = 0; si < n_segs; ++si) {
     const Seg seg = s.segs[si];
     const int nt = h16_tiles(seg);
     if (nt <= 0) continue;
     const int* pt = P.page_table + (long long)seg.b * P.pt_stride;
-    const int tok_base = seg.tok0 + kH16Own * cg;
-    auto fetch_ids = [&](int t, int (&page)[3]) {
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const int tok = tok_base + t * kH16Tile + r[i];
-        page[i] = tok < seg.tok_end ? pt[tok >> P.page_shift] : -1;
-      }
-    };
-    auto fetch_rows = [&](int t, const int (&page)[3], H16Raw& R) {
-      long long row[3];
-      bool live[3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const int tok = tok_base + t * kH16Tile + r[i];
-        live[i] = tok < seg.tok_end;
-        // a stale or corrupt id is never dereferenced: the row reads as zeros and the call is flagged
-        if (live[i] && uint32_t(page[i]) >= uint32_t(P.num_pages)) atomicExch(P.header, int(kBadPage)), live[i] = false;
-        row[i] = ((long long)page[i] << P.page_shift) + (tok & ps_mask);
-      }
+    uint4 rw[2];
+    uint32_t rs[2];
+    uint2 rr[2];
+    int ru[2], rj[2] = {0, 0};           // cache rows of the two latent units and the two rope chunks, negative: none
+    int tok = seg.tok0 + 32 * v + lane;  // this lane's token of the tile being fetched
+    // No load sits behind a branch (it would be waited for where the branches meet, one trip to memory per load instead of
+    // one per tile): tokens past the end look up the last live token's page, dead rows read cache row 0 and are zeroed where
+    // their bytes are used, and the fetches past the last tile are issued like the others.
+    auto fetch_id = [&](int tk) { return __ldg(pt + ((tk < seg.tok_end ? tk : seg.tok_end - 1) >> P.page_shift)); };
+    auto fetch_rows = [&](int page) {
+      const bool live = tok < seg.tok_end, good = uint32_t(page) < uint32_t(P.num_pages);
+      // a stale or corrupt id is never dereferenced: the row reads as zeros and the call is flagged
+      if (live && !good) atomicExch(P.header, int(kBadPage));
+      const int row = live && good ? (page << P.page_shift) + (tok & ((1 << P.page_shift) - 1)) : -1;
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        R.w[u] = make_uint4(0, 0, 0, 0), R.sf[u] = 0;
-        if (live[u]) {
-          R.w[u] = __ldg(reinterpret_cast<const uint4*>(P.ckv + row[u] * 256 + 32 * w + 16 * hh));
-          R.sf[u] = __ldg(reinterpret_cast<const unsigned short*>(P.sf + row[u] * 32 + 4 * w + 2 * hh));
+        ru[u] = __shfl_sync(~0u, row, 16 * u + (lane >> 1));
+        const long long at = ru[u] < 0 ? 0 : ru[u];
+        rw[u] = __ldg(reinterpret_cast<const uint4*>(ckv0 + at * 256));
+        rs[u] = __ldg(reinterpret_cast<const unsigned short*>(sf0 + at * 32));
+      }
+      if constexpr (part_a) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          rj[j] = __shfl_sync(~0u, row, rope_row + 4 * j);
+          rr[j] = __ldg(reinterpret_cast<const uint2*>(kpe0 + (long long)(rj[j] < 0 ? 0 : rj[j]) * 64));
         }
       }
-      R.rope = make_uint2(0, 0);
-      if (live[2]) R.rope = __ldg(reinterpret_cast<const uint2*>(P.kpe + row[2] * 64 + 8 * (lane & 7)));
+      tok += kH16Tile;
     };
-    int page[3];
-    H16Raw raw;
-    fetch_ids(0, page);
-    fetch_rows(0, page, raw);
-    fetch_ids(1, page);
+    fetch_rows(fetch_id(tok));
+    int page = fetch_id(tok);
     for (int t = 0; t < nt; ++t, ++it) {
-      const uint32_t kb = it & 1;
-      uint4 o[2][4], orope;
+      const uint32_t kb = it & 1, buf = kb * uint32_t(sizeof(s.kv[0]));
+      // this part of the buffer was released by the MMAs of tile it - 2
+      if (it >= 2 && !__all_sync(~0u, ptx::mbar_wait(&freed[kb], ((it >> 1) - 1) & 1, &s.abort_flag))) return;
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const uint32_t s2 = ptx::e4m3x2_to_f16x2(uint16_t(raw.sf[u]));  // scales of the unit's two blocks
+        const uint32_t s2 = ru[u] < 0 ? 0u : ptx::e4m3x2_to_f16x2(uint16_t(rs[u]));  // scales of the unit's two blocks
         const uint32_t sc[2] = {__byte_perm(s2, s2, 0x1010), __byte_perm(s2, s2, 0x3232)};
-        const uint32_t words[4] = {raw.w[u].x, raw.w[u].y, raw.w[u].z, raw.w[u].w};
+        const uint32_t words[4] = {rw[u].x, rw[u].y, rw[u].z, rw[u].w};
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           uint32_t e[4];
           ptx::e2m1x8_to_f16x8(words[c], e);
-          o[u][c] = make_uint4(ptx::hmul2(e[0], sc[c >> 1]), ptx::hmul2(e[1], sc[c >> 1]), ptx::hmul2(e[2], sc[c >> 1]), ptx::hmul2(e[3], sc[c >> 1]));
+          ptx::sts128(dst0 + buf + u * 2048 + ((uint32_t(c) << 4) ^ swz), ptx::hmul2(e[0], sc[c >> 1]), ptx::hmul2(e[1], sc[c >> 1]),
+                      ptx::hmul2(e[2], sc[c >> 1]), ptx::hmul2(e[3], sc[c >> 1]));
         }
       }
-      orope = make_uint4(ptx::e4m3x2_to_f16x2(uint16_t(raw.rope.x)), ptx::e4m3x2_to_f16x2(uint16_t(raw.rope.x >> 16)),
-                         ptx::e4m3x2_to_f16x2(uint16_t(raw.rope.y)), ptx::e4m3x2_to_f16x2(uint16_t(raw.rope.y >> 16)));
-      if (t + 1 < nt) fetch_rows(t + 1, page, raw);
-      if (t + 2 < nt) fetch_ids(t + 2, page);
-      // the panel is part B of CTA hf (released by its PV) and part A of the other one (released by its QK^T); the rope
-      // panel is part A of both
-      if (it >= 2) {
-        const uint32_t ph = ((it >> 1) - 1) & 1;
-        bool ok = ptx::mbar_wait(&s.free_a[hf ^ 1][kb], ph, &s.abort_flag) && ptx::mbar_wait(&s.free_a[hf][kb], ph, &s.abort_flag);
-        ok = ok && ptx::mbar_wait(&s.free_b[hf][kb], ph, &s.abort_flag);
-        if (!__all_sync(~0u, ok)) return;
-      }
+      if constexpr (part_a) {
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        uint8_t* out_row = s.kv[kb][w] + (kH16Own * cg + r[u]) * 128;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(out_row + (uint32_t((4 * hh + c) ^ (r[u] & 7)) << 4)) = o[u][c];
+        for (int j = 0; j < 2; ++j) {
+          const uint2 x = rj[j] < 0 ? make_uint2(0, 0) : rr[j];
+          ptx::sts128(rope0 + buf + j * 512 + ((rope_c ^ (rope_s + 4 * j)) << 4), ptx::e4m3x2_to_f16x2(uint16_t(x.x)),
+                      ptx::e4m3x2_to_f16x2(uint16_t(x.x >> 16)), ptx::e4m3x2_to_f16x2(uint16_t(x.y)), ptx::e4m3x2_to_f16x2(uint16_t(x.y >> 16)));
+        }
       }
-      *reinterpret_cast<uint4*>(s.kv[kb][8] + (kH16Own * cg + r[2]) * 128 + (uint32_t((lane & 7) ^ (r[2] & 7)) << 4)) = orope;
       ptx::fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) {
-        // the peer's tile gets the same bytes; they complete on its barrier of the part they belong to
-        const uint8_t* src = s.kv[kb][w] + kH16Own * cg * 128;
-        const uint8_t* rsrc = s.kv[kb][8] + (kH16Own * cg + 4 * w) * 128;
-        uint64_t* peer_full = uint32_t(hf) == peer ? &s.full_b[kb] : &s.full_a[kb];
-        ptx::bulk_copy_to_cta(ptx::map_to_cta(src, peer), src, 4096, ptx::map_to_cta(peer_full, peer));
-        ptx::bulk_copy_to_cta(ptx::map_to_cta(rsrc, peer), rsrc, 512, ptx::map_to_cta(&s.full_a[kb], peer));
-        if (w == 0) ptx::mbar_arrive_expect_tx(&s.full_a[kb], kH16PeerA);  // what the peer will send for this tile
-        else ptx::mbar_arrive(&s.full_a[kb]);
-        if (hf == cg) {
-          if ((w & 3) == 0) ptx::mbar_arrive_expect_tx(&s.full_b[kb], kH16PeerB);
-          else ptx::mbar_arrive(&s.full_b[kb]);
-        }
-        if (w == 0) s.progress = it + 1;
-      }
-      __syncwarp();
+      ptx::mbar_arrive_if(&full[kb], lane == 0);
+      if (cw == 0 && lane == 0) s.progress = it + 1;
+      const int pg = page;
+      page = fetch_id(tok + kH16Tile);
+      fetch_rows(pg);
     }
   }
+}
+
+__device__ __forceinline__ void h16_convert_role(H16Smem& s, const DecodeParams& P, int n_segs, uint32_t& it, int cg) {
+  if (int(((threadIdx.x >> 5) - 8) >> 2 & 1) != cg) h16_convert_warps<true>(s, P, n_segs, it);
+  else h16_convert_warps<false>(s, P, n_segs, it);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -240,9 +230,10 @@ __device__ __forceinline__ void h16_convert_role(H16Smem& s, const DecodeParams&
 // ---------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void h16_qk_role(H16Smem& s, const DecodeParams& P, int n_segs, uint32_t& it, uint32_t& seg_count, int cg) {
   const bool leader = ptx::elect_one();
-  const uint32_t tm = s.tmem_base;
+  const uint32_t tm = 0;  // all 512 columns are allocated: they start at column 0 (a constant keeps the MMA operands uniform)
   const uint32_t idesc = ptx::instr_desc(kH16Rows, kH16Tile, ptx::FMT_F16, ptx::FMT_F16, false, false);
-  const uint64_t q_desc = ptx::smem_desc_sw128(ptx::smem_u32(s.q[0]), 16, 1024);
+  const uint64_t q_desc = ptx::smem_desc_sw128(ptx::smem_u32(s.q[0]), 16, 1024), kv_desc = ptx::smem_desc_sw128(ptx::smem_u32(s.kv[0][0]), 16, 1024);
+  const uint32_t hi = uint32_t(q_desc >> 32);
   for (int si = 0; si < n_segs; ++si) {
     const int nt = h16_tiles(s.segs[si]);
     if (nt <= 0) continue;
@@ -250,38 +241,36 @@ __device__ __forceinline__ void h16_qk_role(H16Smem& s, const DecodeParams& P, i
     ++seg_count;
     for (int t = 0; t < nt; ++t, ++it) {
       const uint32_t kb = it & 1;
-      const uint64_t k_desc = ptx::smem_desc_sw128(ptx::smem_u32(s.kv[kb][0]), 16, 1024);
+      const uint32_t k_lo = uint32_t(kv_desc) + kb * uint32_t(sizeof(s.kv[0]) >> 4);
       // the four latent panels of one half: channels [0, 256) have Q in tensor memory, [256, 512) in shared memory
       auto half = [&](int h, uint32_t accum) {
+        uint32_t q = h == 0 ? tm + H16Cols::QN : uint32_t(q_desc), k = k_lo + h * (4 * kH16Panel >> 4);
         if (h == 0) {
 #pragma unroll 1
-          for (int k = 0; k < 16; ++k)
-            ptx::mma_f16_ts(tm + H16Cols::S, tm + H16Cols::QN + 8 * k, k_desc + (((k >> 2) * kH16Panel + (k & 3) * 32) >> 4), idesc, accum | k);
+          for (int p = 0; p < 4; ++p, q += 32, k += kH16Panel >> 4)
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) ptx::mma_f16_ts_if(leader, tm + H16Cols::S, q + 8 * ks, k + 2 * ks, hi, idesc, ks ? 1u : accum | p);
         } else {
 #pragma unroll 1
-          for (int k = 0; k < 16; ++k)
-            ptx::mma_f16_ss(tm + H16Cols::S, q_desc + (((k >> 2) * (kH16Rows * 128) + (k & 3) * 32) >> 4),
-                            k_desc + (((4 + (k >> 2)) * kH16Panel + (k & 3) * 32) >> 4), idesc, accum | k);
+          for (int p = 0; p < 4; ++p, q += kH16Rows * 128 >> 4, k += kH16Panel >> 4)
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) ptx::mma_f16_ss_if(leader, tm + H16Cols::S, q + 2 * ks, k + 2 * ks, hi, idesc, ks ? 1u : accum | p);
         }
       };
       // the softmax warps have read the scores of tile it - 1; part A of this tile is in place
       if (!__all_sync(~0u, it < 1 || ptx::mbar_wait(&s.s_free, (it - 1) & 1, &s.abort_flag))) return;
       if (!__all_sync(~0u, ptx::mbar_wait(&s.full_a[kb], (it >> 1) & 1, &s.abort_flag))) return;
       ptx::tc_fence_after_sync();
-      if (leader) {
-        half(cg ^ 1, 0);
+      half(cg ^ 1, 0u);
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          ptx::mma_f16_ts(tm + H16Cols::S, tm + H16Cols::QR + 8 * ks, k_desc + ((8 * kH16Panel + ks * 32) >> 4), idesc, 1);
-        ptx::mma_commit_pair(&s.free_a[cg][kb]);
-      }
+      for (int ks = 0; ks < 4; ++ks)
+        ptx::mma_f16_ts_if(leader, tm + H16Cols::S, tm + H16Cols::QR + 8 * ks, k_lo + ((8 * kH16Panel + ks * 32) >> 4), hi, idesc, 1u);
+      if (leader) ptx::mma_commit(&s.free_a[kb]);
       __syncwarp();
       if (!__all_sync(~0u, ptx::mbar_wait(&s.full_b[kb], (it >> 1) & 1, &s.abort_flag))) return;
       ptx::tc_fence_after_sync();
-      if (leader) {
-        half(cg, 1);
-        ptx::mma_commit(&s.s_full);
-      }
+      half(cg, 1u);
+      if (leader) ptx::mma_commit(&s.s_full);
       __syncwarp();
     }
   }
@@ -289,7 +278,7 @@ __device__ __forceinline__ void h16_qk_role(H16Smem& s, const DecodeParams& P, i
 
 __device__ __forceinline__ void h16_pv_role(H16Smem& s, const DecodeParams& P, int n_segs, uint32_t& it, int cg) {
   const bool leader = ptx::elect_one();
-  const uint32_t tm = s.tmem_base;
+  const uint32_t tm = 0;  // all 512 columns are allocated: they start at column 0 (a constant keeps the MMA operands uniform)
   // B = V read MN-major: N = 256 channels = four 128-byte runs (panels 4 cg .. 4 cg + 3), K = 16 token rows
   const uint32_t idesc = ptx::instr_desc(kH16Rows, 256, ptx::FMT_F16, ptx::FMT_F16, false, true);
   for (int si = 0; si < n_segs; ++si) {
@@ -298,13 +287,13 @@ __device__ __forceinline__ void h16_pv_role(H16Smem& s, const DecodeParams& P, i
       const uint32_t kb = it & 1;
       if (!__all_sync(~0u, ptx::mbar_wait(&s.p_full, it & 1, &s.abort_flag))) return;
       ptx::tc_fence_after_sync();
-      if (leader) {
-        const uint64_t v_desc = ptx::smem_desc_sw128(ptx::smem_u32(s.kv[kb][4 * cg]), kH16Panel, 1024);
+      const uint64_t v_desc = ptx::smem_desc_sw128(ptx::smem_u32(s.kv[kb][4 * cg]), kH16Panel, 1024);
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          ptx::mma_f16_ts(tm + H16Cols::O, tm + H16Cols::P + 8 * ks, v_desc + ((ks * 16 * 128) >> 4), idesc, (t | ks) != 0);
+      for (int ks = 0; ks < 4; ++ks)
+        ptx::mma_f16_ts_if(leader, tm + H16Cols::O, tm + H16Cols::P + 8 * ks, uint32_t(v_desc) + ((ks * 16 * 128) >> 4), uint32_t(v_desc >> 32), idesc, (t | ks) != 0);
+      if (leader) {
         ptx::mma_commit(&s.pv_done);
-        ptx::mma_commit_pair(&s.free_b[cg][kb]);
+        ptx::mma_commit(&s.free_b[kb]);
       }
       __syncwarp();
     }
@@ -352,92 +341,66 @@ __device__ __forceinline__ void h16_softmax_role(H16Smem& s, const DecodeParams&
 #pragma unroll
     for (int l = 0; l < 4; ++l) ptx::prefetch_l2(reinterpret_cast<const char*>(qn) + 128 * l);
     if (half) ptx::prefetch_l2(qp);
-    // largest magnitude, as BF16 bits (ordered like integers); an infinity or NaN shows as >= 0x7F80
-    auto amax_bits = [](const uint4* src, int n) {
-      uint32_t m2 = 0;
-#pragma unroll 1
-      for (int c0 = 0; c0 < n; c0 += 8) {
-        uint4 v[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) v[c] = __ldg(src + c0 + c);
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          m2 = ptx::max_s16x2(ptx::max_s16x2(m2, ptx::max_s16x2(v[c].x & 0x7FFF7FFFu, v[c].y & 0x7FFF7FFFu)),
-                              ptx::max_s16x2(v[c].z & 0x7FFF7FFFu, v[c].w & 0x7FFF7FFFu));
-      }
-      return max(m2 & 0xFFFFu, m2 >> 16);
-    };
-    // non-finite elements become 0: they have no meaningful result anyway, the rest of the row stays intact
-    auto clean = [](uint32_t x) {
-      if ((x & 0x7F80u) == 0x7F80u) x &= 0xFFFF0000u;
-      if ((x & 0x7F800000u) == 0x7F800000u) x &= 0x0000FFFFu;
-      return x;
-    };
-    uint32_t bits = amax_bits(qn, 32), bits_p = half ? amax_bits(qp, KPE / 8) : 0u;
-    const bool odd = bits >= 0x7F80u || bits_p >= 0x7F80u;
-    if (odd) {  // once more, without the non-finite ones
-      bits = bits_p = 0;
-      auto fold = [&](const uint4& v, uint32_t m) {
-        const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint32_t c = clean(wv[j]) & 0x7FFF7FFFu;
-          m = max(m, max(c & 0xFFFFu, c >> 16));
-        }
-        return m;
+    // Q as FP16 times `up`, into tensor memory / shared memory; returns the largest magnitude of the finite elements (the rope part
+    // times `ratio`). Non-finite elements become 0: they have no meaningful result anyway, the rest of the row stays intact.
+    auto load_query = [&](float up) {
+      uint32_t m2 = 0, m2p = 0;  // BF16 magnitudes, two at a time, ordered like integers
+      auto clean = [](uint32_t x) {
+        if ((x & 0x7F80u) == 0x7F80u) x &= 0xFFFF0000u;
+        if ((x & 0x7F800000u) == 0x7F800000u) x &= 0x0000FFFFu;
+        return x;
+      };
+      auto two = [&](uint32_t x, float sc, uint32_t& mm) {
+        x = clean(x);
+        mm = ptx::max_s16x2(mm, x & 0x7FFF7FFFu);
+        return ptx::f32x2_to_f16x2(__uint_as_float(x << 16) * sc, __uint_as_float(x & 0xFFFF0000u) * sc);
       };
 #pragma unroll 1
-      for (int c = 0; c < 32; ++c) bits = fold(qn[c], bits);
-      if (half)
-#pragma unroll 1
-        for (int c = 0; c < KPE / 8; ++c) bits_p = fold(qp[c], bits_p);
-    }
-    s.xch[half][h] = fmaxf(__uint_as_float(bits << 16), __uint_as_float(bits_p << 16) * ratio);
-    ptx::bar_sync(pair_bar, 64);
-    // the row is scaled by 2^(14 - e), e = floor(log2(row maximum)): FP16 then holds a BF16 element exactly down to 2^-29 of
-    // the maximum. The sign of the softmax scale goes into Q, so that a larger accumulator is always a larger score.
-    int e = int(__float_as_uint(fmaxf(s.xch[0][h], s.xch[1][h])) >> 23) - 127;
-    e = e < -80 ? -80 : e > 126 ? 126 : e;
-    float up = __uint_as_float(uint32_t(14 - e + 127) << 23);
-    const float qa = fmaxf(fabsf(P.sm_scale_log2) * P.ckv_scale * __uint_as_float(uint32_t(e - 14 + 127) << 23), 1e-37f);
-    up = P.sm_scale_log2 < 0.f ? -up : up;
-    auto f16x8 = [&](uint4 v, float sc) {
-      if (odd) v = make_uint4(clean(v.x), clean(v.y), clean(v.z), clean(v.w));
-      auto two = [&](uint32_t x) { return ptx::f32x2_to_f16x2(__uint_as_float(x << 16) * sc, __uint_as_float(x & 0xFFFF0000u) * sc); };
-      return make_uint4(two(v.x), two(v.y), two(v.z), two(v.w));
-    };
-#pragma unroll 1
-    for (int c0 = 0; c0 < 32; c0 += 8) {  // 64 channels per trip
-      uint4 v[8];
+      for (int c0 = 0; c0 < 32; c0 += 8) {  // 64 channels per trip
+        uint4 v[8];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) v[c] = __ldg(qn + c0 + c);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) v[c] = f16x8(v[c], up);
-      if (half == 0) {
+        for (int c = 0; c < 8; ++c) v[c] = __ldg(qn + c0 + c);
         uint32_t col[32];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) col[4 * c] = v[c].x, col[4 * c + 1] = v[c].y, col[4 * c + 2] = v[c].z, col[4 * c + 3] = v[c].w;
-        ptx::tmem_st32(tm_lane + H16Cols::QN + 4 * c0, col);
-      } else {
-        uint8_t* dst = s.q[c0 >> 3] + h * 128;
+        for (int c = 0; c < 8; ++c)
+          col[4 * c] = two(v[c].x, up, m2), col[4 * c + 1] = two(v[c].y, up, m2), col[4 * c + 2] = two(v[c].z, up, m2), col[4 * c + 3] = two(v[c].w, up, m2);
+        if (half == 0) {
+          ptx::tmem_st32(tm_lane + H16Cols::QN + 4 * c0, col);
+        } else {
+          const uint32_t dst = ptx::smem_u32(s.q[c0 >> 3]) + h * 128;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(dst + (uint32_t(c ^ (h & 7)) << 4)) = v[c];
+          for (int c = 0; c < 8; ++c) ptx::sts128(dst + (uint32_t(c ^ (h & 7)) << 4), col[4 * c], col[4 * c + 1], col[4 * c + 2], col[4 * c + 3]);
+        }
       }
-    }
-    if (half) {
-      uint32_t col[32];
+      if (half) {
+        uint32_t col[32];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        uint4 v = __ldg(qp + c);
-        if (odd) v = make_uint4(clean(v.x), clean(v.y), clean(v.z), clean(v.w));
-        const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          col[4 * c + j] = ptx::f32x2_to_f16x2(__uint_as_float(wv[j] << 16) * ratio * up, __uint_as_float(wv[j] & 0xFFFF0000u) * ratio * up);
+        for (int c = 0; c < 8; ++c) {
+          const uint4 v = __ldg(qp + c);
+          col[4 * c] = two(v.x, up * ratio, m2p), col[4 * c + 1] = two(v.y, up * ratio, m2p), col[4 * c + 2] = two(v.z, up * ratio, m2p), col[4 * c + 3] = two(v.w, up * ratio, m2p);
+        }
+        ptx::tmem_st32(tm_lane + H16Cols::QR, col);
       }
-      ptx::tmem_st32(tm_lane + H16Cols::QR, col);
-      ptx::fence_proxy_async_smem();
+      return fmaxf(__uint_as_float(max(m2 << 16, m2 & 0xFFFF0000u)), __uint_as_float(max(m2p << 16, m2p & 0xFFFF0000u)) * ratio);
+    };
+    // The sign of the softmax scale goes into Q, so that a larger accumulator is always a larger score. FP16 holds the BF16
+    // elements of an ordinary row as they are (exactly from 2^-14 up, to 2^-24 below: 2^-16 of the row's maximum at worst): one
+    // pass over it. A row whose maximum lies outside [2^-8, 2^14] is loaded again times a power of two that puts its maximum
+    // into [2^14, 2^15); the tensor-memory stores are warp-wide, so the pair of warps decides together.
+    const float sign = P.sm_scale_log2 < 0.f ? -1.f : 1.f;
+    s.xch[half][h] = load_query(sign);
+    ptx::bar_sync(pair_bar, 64);
+    const float amax = fmaxf(s.xch[0][h], s.xch[1][h]);
+    float down = 1.f;  // what the scores are to be multiplied with
+    const bool ordinary = amax >= 0x1p-8f && amax <= 0x1p14f;
+    if (!__all_sync(~0u, ordinary)) {  // (both warps of the pair see the same maxima)
+      int e = int(__float_as_uint(amax) >> 23) - 127 - 14;
+      e = ordinary ? 0 : e < -94 ? -94 : e > 112 ? 112 : e;
+      load_query(sign * __uint_as_float(uint32_t(127 - e) << 23));
+      down = __uint_as_float(uint32_t(127 + e) << 23);
     }
+    const float qa = fmaxf(fabsf(P.sm_scale_log2) * P.ckv_scale * down, 1e-37f);
+    if (half) ptx::fence_proxy_async_smem();
     ptx::tmem_wait_st();
     ptx::tc_fence_before_sync();
     __syncwarp();
@@ -495,14 +458,15 @@ __device__ __forceinline__ void h16_softmax_role(H16Smem& s, const DecodeParams&
       // P = 2^(s qa - m) as FP16 into this warp's 16 of the tile's 32 P columns, once PV of tile it - 1 has read them
       const float neg_m = (m == -INFINITY) ? 0.f : -m;
       uint32_t pk[16];
-      float ls[4] = {0.f, 0.f, 0.f, 0.f};
+      float2 ls[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
       for (int c = 0; c < 16; ++c) {
-        const float p0 = ptx::ex2(fmaf(__uint_as_float(sr[2 * c]), qa, neg_m)), p1 = ptx::ex2(fmaf(__uint_as_float(sr[2 * c + 1]), qa, neg_m));
-        ls[c & 3] += p0 + p1;
-        pk[c] = ptx::f32x2_to_f16x2(p0, p1);
+        const float2 x = ptx::fma_f32x2(make_float2(__uint_as_float(sr[2 * c]), __uint_as_float(sr[2 * c + 1])), make_float2(qa, qa), make_float2(neg_m, neg_m));
+        const float2 p = make_float2(ptx::ex2(x.x), ptx::ex2(x.y));
+        ls[c & 1] = ptx::add_f32x2(ls[c & 1], p);
+        pk[c] = ptx::f32x2_to_f16x2(p.x, p.y);
       }
-      l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+      l += (ls[0].x + ls[0].y) + (ls[1].x + ls[1].y);
       if (it >= 1) {  // (a wait that gives up raises the abort flag; the next vote or the epilogue ends the role for both warps)
         ptx::mbar_wait(&s.pv_done, (it - 1) & 1, &s.abort_flag);
         ptx::tc_fence_after_sync();
@@ -568,12 +532,6 @@ __device__ __forceinline__ void h16_run_role(H16Smem& s, const DecodeParams& P) 
     __syncthreads();
     if (s.abort_flag) break;
   }
-  // The releases of the last two tiles come from the peer as well: see them arrive before this CTA's memory goes away. (The
-  // convert warps have seen those of all earlier tiles, so each barrier is at most one phase short.)
-  if (ROLE == kH16Prefetch && !s.abort_flag)
-    for (uint32_t j = it >= 2 ? it - 2 : 0; j < it; ++j)
-      for (int x = 0; x < 2; ++x)
-        ptx::mbar_wait(&s.free_a[x][j & 1], (j >> 1) & 1, &s.abort_flag), ptx::mbar_wait(&s.free_b[x][j & 1], (j >> 1) & 1, &s.abort_flag);
 }
 
 __global__ void __launch_bounds__(kH16Threads, 1) mla_decode_hm16_kernel(const DecodeParams P) {
@@ -583,8 +541,8 @@ __global__ void __launch_bounds__(kH16Threads, 1) mla_decode_hm16_kernel(const D
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
-      ptx::mbar_init(&s.full_a[i], 8), ptx::mbar_init(&s.full_b[i], 4);
-      for (int x = 0; x < 2; ++x) ptx::mbar_init(&s.free_a[x][i], 1), ptx::mbar_init(&s.free_b[x][i], 1);
+      ptx::mbar_init(&s.full_a[i], 8), ptx::mbar_init(&s.full_b[i], 8);
+      ptx::mbar_init(&s.free_a[i], 1), ptx::mbar_init(&s.free_b[i], 1);
     }
     ptx::mbar_init(&s.s_full, 1), ptx::mbar_init(&s.s_free, 8);
     ptx::mbar_init(&s.p_full, 8), ptx::mbar_init(&s.pv_done, 1);
@@ -592,38 +550,38 @@ __global__ void __launch_bounds__(kH16Threads, 1) mla_decode_hm16_kernel(const D
     s.abort_flag = 0, s.progress = 0;
     ptx::fence_mbar_init();
   }
-  if (warp == 16) {
+  if (warp == 24) {
     ptx::tmem_alloc(&s.tmem_base, kTmemCols);
     ptx::tmem_relinquish();
   }
   ptx::tc_fence_before_sync();
-  ptx::cluster_sync();  // both CTAs' barriers are initialised before either signals the other's
+  __syncthreads();
   ptx::tc_fence_after_sync();
   ptx::grid_dependency_wait();
   ptx::grid_launch_dependents();  // after the wait: the combine kernel reads a schedule kernel's output as soon as it starts
-  // the query panels are written by this CTA's own softmax warps only (the peer writes to kv): free until then
+  // the query panels are free until the softmax warps write them
   if (P.inline_sched) publish_own_schedule<kH16Threads>(reinterpret_cast<int*>(s.q[0]), P, blockIdx.x >> 1);
 
-  // register budgets, warp group by warp group; the pool is the launch allocation, 20 warps x 96
-  constexpr int kLaunchRegs = 96, kSoftmaxRegs = 104, kConvertRegs = 112, kIssueRegs = 48;
-  static_assert(8 * kSoftmaxRegs + 8 * kConvertRegs + 4 * kIssueRegs <= 20 * kLaunchRegs, "register budgets exceed the CTA's allocation");
+  // register budgets, warp group by warp group; the pool is the launch allocation, 28 warps x 72
+  constexpr int kLaunchRegs = 72, kSoftmaxRegs = 96, kConvertRegs = 64, kIssueRegs = 48;
+  static_assert(8 * kSoftmaxRegs + 16 * kConvertRegs + 4 * kIssueRegs <= 28 * kLaunchRegs, "register budgets exceed the CTA's allocation");
   if (warp < 8) {
     ptx::reg_alloc<kSoftmaxRegs>();
     h16_run_role<kH16Softmax>(s, P);
-  } else if (warp < 16) {
-    ptx::reg_alloc<kConvertRegs>();
+  } else if (warp < 24) {
+    ptx::reg_dealloc<kConvertRegs>();
     h16_run_role<kH16Convert>(s, P);
   } else {
     ptx::reg_dealloc<kIssueRegs>();
-    if (warp == 16) h16_run_role<kH16Qk>(s, P);
-    else if (warp == 17) h16_run_role<kH16Prefetch>(s, P);
-    else if (warp == 18) h16_run_role<kH16Pv>(s, P);
+    if (warp == 24) h16_run_role<kH16Qk>(s, P);
+    else if (warp == 25) h16_run_role<kH16Prefetch>(s, P);
+    else if (warp == 26) h16_run_role<kH16Pv>(s, P);
     else h16_run_role<kH16Idle>(s, P);
   }
 
   ptx::tc_fence_before_sync();
-  ptx::cluster_sync();  // neither CTA leaves while the other may still write to its shared memory or signal its barriers
-  if (warp == 16) ptx::tmem_dealloc(s.tmem_base, kTmemCols);
+  __syncthreads();
+  if (warp == 24) ptx::tmem_dealloc(s.tmem_base, kTmemCols);
   if (threadIdx.x == 0 && s.abort_flag) atomicExch(P.header, int(kWaitTimeout));
 }
 

@@ -86,6 +86,9 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(d.x), "=r"(d.y), "=r"(d.z), "=r"(d.w) : "r"(addr));
   return d;
 }
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 __device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 
 // Split form of the bounded wait, for a barrier that has usually completed by the time it is needed: mbar_probe()
@@ -320,6 +323,27 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accum)
       : "memory");
 }
+// The same two, issued by the one thread of the warp whose `lead` is set, without a branch, and with the operand descriptors
+// as their low words (start address and LBO; a K step or panel is one 32-bit addition) plus a constant high word: fewer
+// registers and instructions per MMA where a warp issues dozens of short ones per tile.
+__device__ __forceinline__ void mma_f16_ss_if(uint32_t lead, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc,
+                                              uint32_t accum) {
+  asm volatile(
+      "{\n.reg .pred p, q;\n.reg .b64 da, db;\nsetp.ne.b32 p, %5, 0;\nsetp.ne.b32 q, %6, 0;\n"
+      "mov.b64 da, {%1, %3};\nmov.b64 db, {%2, %3};\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accum), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void mma_f16_ts_if(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc,
+                                              uint32_t accum) {
+  asm volatile(
+      "{\n.reg .pred p, q;\n.reg .b64 db;\nsetp.ne.b32 p, %5, 0;\nsetp.ne.b32 q, %6, 0;\n"
+      "mov.b64 db, {%2, %3};\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accum), "r"(lead)
+      : "memory");
+}
 __device__ __forceinline__ void mma_f8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accum) {
   asm volatile(
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
@@ -354,12 +378,6 @@ __device__ __forceinline__ void mma_mxf4nvf4_ss(uint32_t d_tmem, uint64_t a_desc
 // mbarrier arrives once every tcgen05 operation this thread issued so far has completed
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// the same on the mbarrier at this offset in BOTH CTAs of a cluster of two
-__device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "h"(uint16_t(3))
-               : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -446,6 +464,22 @@ __device__ __forceinline__ uint32_t max_s16x2(uint32_t a, uint32_t b) {
 __device__ __forceinline__ float max3(float a, float b, float c) {  // one instruction on sm_100
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// packed fp32: both lanes in one instruction
+__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\n"
+      "fma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
 __device__ __forceinline__ float ex2(float x) {

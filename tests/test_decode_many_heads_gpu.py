@@ -17,17 +17,17 @@ pytestmark = pytest.mark.gpu
 LN2 = math.log(2.0)
 
 
-def run(c, sm_scale=SM_SCALE, num_splits=0):
+def run(c, sm_scale=SM_SCALE, num_splits=0, longest=1 << 20):
+    # a high bound of the lengths selects the kernel, however short they are
     args = (c.q_nope, c.q_pe, c.ckv_cache, c.ckv_sf_cache, c.kpe_cache, c.page_table, c.kv_lens, sm_scale, c.ckv_scale, c.kpe_scale)
-    longest = max(c.kv_lens_list)
     out = mla.decode(*args, max_kv_len=longest, num_splits=num_splits)
     _, lse2 = mla.decode_partial(*args, max_kv_len=longest, num_splits=num_splits)
     assert mla.workspace_status() == 0
     return out.float().cpu().numpy(), lse2.cpu().numpy() * LN2
 
 
-def check(c, sm_scale=SM_SCALE, num_splits=0):
-    got, lse = run(c, sm_scale, num_splits)
+def check(c, sm_scale=SM_SCALE, num_splits=0, longest=1 << 20):
+    got, lse = run(c, sm_scale, num_splits, longest)
     want, want_lse = oracle_reference(c, sm_scale)
     live = [b for b, n in enumerate(c.kv_lens_list) if n > 0]
     assert np.abs(got - want).max() <= 2e-2
@@ -41,7 +41,7 @@ def check(c, sm_scale=SM_SCALE, num_splits=0):
 @pytest.mark.parametrize("heads", [64, 80, 112, 128, 144, 192, 256])
 @pytest.mark.parametrize("num_splits", [0, 3])
 def test_head_groups(heads, num_splits):
-    check(SyntheticCache([513, 64, 1], 64, heads, None, None, seed=heads).to("cuda"), num_splits=num_splits)
+    check(SyntheticCache([5000, 513, 64, 1], 64, heads, None, None, seed=heads).to("cuda"), num_splits=num_splits, longest=5000)
 
 
 @pytest.mark.parametrize("page_size", [1, 2, 8, 16, 32, 64, 256])
@@ -64,6 +64,8 @@ def test_wide_range_of_query_magnitudes_and_non_finite_elements():
     c = SyntheticCache([500, 129], 64, 64, 0.01, 0.01, seed=2).to("cuda")
     c.q_nope[:, :, 7] *= 64.0                       # outlier channel
     c.q_nope[:, 3] *= 2.0 ** -60                    # a tiny row
+    c.q_nope[:, 9] *= 2.0 ** -60
+    c.q_pe[:, 9] *= 2.0 ** -60
     c.q_pe[:, 5] *= 32.0                            # the rope part decides the row's scale
     check(c)
     clean, _ = run(c)
@@ -80,12 +82,21 @@ def test_wide_range_of_query_magnitudes_and_non_finite_elements():
     assert np.array_equal(got, zeroed)
 
 
+def test_both_sides_of_the_dispatch_agree():
+    """64 heads, ten requests: a bound of 14 tiles per request is the last one of the 16-head kernel on 148 SMs, 15 the first of
+    this one."""
+    c = SyntheticCache([400] * 10, 64, 64, None, None, seed=8).to("cuda")
+    few, few_lse = run(c, longest=14 * 128)
+    many, many_lse = run(c, longest=15 * 128)
+    assert O.rel_l2(few, many) < 4e-3 and np.abs(few_lse - many_lse).max() <= 1e-3
+
+
 @pytest.mark.parametrize("page_size", [16, 64])
 def test_page_ids_are_range_checked(page_size):
     c = SyntheticCache([200, 90], page_size, 128, None, None, seed=4).to("cuda")
     good, _ = run(c)
     c.page_table[1, 0] = c.ckv_cache.shape[0] + 5
     args = (c.q_nope, c.q_pe, c.ckv_cache, c.ckv_sf_cache, c.kpe_cache, c.page_table, c.kv_lens, SM_SCALE, c.ckv_scale, c.kpe_scale)
-    out = mla.decode(*args, max_kv_len=200)
+    out = mla.decode(*args, max_kv_len=1 << 20)
     assert mla.workspace_status(clear=True) == 3
     assert np.array_equal(out[0].float().cpu().numpy(), good[0]) and torch.isfinite(out.float()).all()
