@@ -53,7 +53,8 @@ def _workspace(device, stream, nbytes):
 
 
 def _decode(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_table, kv_lens, sm_scale, ckv_scale, kpe_scale,
-            max_kv_len, num_splits, precision, want_out, want_partial, partial_into=None):
+            max_kv_len, num_splits, precision, want_out, want_partial, partial_into=None, q_len=1):
+    # q_len > 1: dimension 1 of the queries holds the heads of q_len query tokens, token by token
     _check_cache(ckv_cache, ckv_sf_cache, kpe_cache)
     if q_nope.dim() != 3 or q_nope.shape[2] != CKV:
         raise RuntimeError("q_nope must be [batch, heads, 512]")
@@ -95,9 +96,10 @@ def _decode(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_table, kv_len
         else:
             o32 = torch.empty(B, H, CKV, dtype=torch.float32, device=dev) if want_partial else None
             lse = torch.empty(B, H, dtype=torch.float32, device=dev) if want_partial else None
-        _lib.check(lib.nvfp4_mla_decode(
+        fn, rows = (lib.nvfp4_mla_decode, (H,)) if q_len == 1 else (lib.nvfp4_mla_decode_multi, (q_len, H // q_len))
+        _lib.check(fn(
             _ptr(q_nope), _ptr(q_pe), _ptr(ckv_cache), _ptr(ckv_sf_cache), _ptr(kpe_cache), ckv_cache.shape[0], ps,
-            _ptr(page_table), page_table.stride(0), _ptr(kv_lens), B, H, float(sm_scale), float(ckv_scale),
+            _ptr(page_table), page_table.stride(0), _ptr(kv_lens), B, *rows, float(sm_scale), float(ckv_scale),
             float(kpe_scale), int(max_kv_len), int(num_splits), int(precision), _ptr(out), _ptr(o32), _ptr(lse),
             _ptr(ws), ws.numel(), stream))
     return out, o32, lse

@@ -291,12 +291,12 @@ int64_t nvfp4_mla_decode_workspace_bytes(int batch, int heads, int num_splits) {
   return a < 0 || b < 0 ? -1 : (a > b ? a : b);
 }
 
-// The decode call proper; `hpc_limit` caps the heads per CTA (see heads_per_cta).
+// The decode call proper; `heads` counts the rows of all q_len query tokens of a request, `hpc_limit` caps the heads per CTA (see heads_per_cta).
 static int decode_impl(const void* q_nope, const void* q_pe, const uint8_t* ckv_cache, const uint8_t* ckv_sf_cache,
                        const uint8_t* kpe_cache, int64_t num_pages, int page_size, const int32_t* page_table,
                        int64_t page_table_stride, const int32_t* kv_lens, int batch, int heads, float sm_scale, float ckv_scale,
                        float kpe_scale, int max_kv_len, int num_splits, int precision, void* out, float* out_f32, float* lse,
-                       void* workspace, int64_t workspace_bytes, void* stream, int hpc_limit) {
+                       void* workspace, int64_t workspace_bytes, void* stream, int hpc_limit, int q_len = 1) {
   g_error[0] = 0;
   MLA_CHECK(precision == NVFP4_MLA_PRECISION_BF16 || precision == NVFP4_MLA_PRECISION_FP8,
             "precision must be 0 (bf16) or 1 (fp8), got %d", precision);
@@ -319,6 +319,8 @@ static int decode_impl(const void* q_nope, const void* q_pe, const uint8_t* ckv_
   MLA_CHECK(workspace_bytes >= int64_t(L.total), "workspace too small: %lld bytes given, %lld needed", (long long)workspace_bytes,
             (long long)L.total);
 
+  MLA_CHECK(q_len == 1 || (hpc > 16 && precision != NVFP4_MLA_PRECISION_FP8),
+            "%d query tokens of %d heads do not share one pass over the cache: decode them as requests", q_len, heads / q_len);
   const bool hm16 = precision != NVFP4_MLA_PRECISION_FP8 && hpc > 16;  // loads with plain instructions: no tensor maps
   CUtensorMap ckv_map, sf_map, kpe_map;
   const int slot_rows = hpc == 128 ? mla::kHmRows : mla::HALF;  // tokens per staging slot of the kernel that will run
@@ -346,7 +348,7 @@ static int decode_impl(const void* q_nope, const void* q_pe, const uint8_t* ckv_
   mla::DecodeParams P;
   P.q_nope = static_cast<const __nv_bfloat16*>(q_nope), P.q_pe = static_cast<const __nv_bfloat16*>(q_pe);
   P.ckv = ckv_cache, P.sf = ckv_sf_cache, P.kpe = kpe_cache, P.page_table = page_table, P.pt_stride = page_table_stride;
-  P.page_shift = __builtin_ctz(unsigned(page_size)), P.num_pages = int(num_pages), P.heads = heads, P.heads_per_cta = hpc;
+  P.page_shift = __builtin_ctz(unsigned(page_size)), P.num_pages = int(num_pages), P.heads = heads, P.heads_per_cta = hpc, P.q_len = q_len;
   P.sf_swz_mask = page_size >= slot_rows ? 1u : 0u, P.kpe_swz_mask = page_size >= slot_rows ? 3u : 0u;
   P.sm_scale_log2 = sm_scale * 1.4426950408889634f, P.ckv_scale = ckv_scale, P.kpe_scale = kpe_scale;
   P.cta_range = cta_range, P.segs = segs, P.lse_part = lse_part, P.o_part = o_part, P.header = header;
@@ -385,6 +387,27 @@ int nvfp4_mla_decode(const void* q_nope, const void* q_pe, const uint8_t* ckv_ca
   return decode_impl(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, num_pages, page_size, page_table, page_table_stride, kv_lens,
                      batch, heads, sm_scale, ckv_scale, kpe_scale, max_kv_len, num_splits, precision, out, out_f32, lse, workspace,
                      workspace_bytes, stream, 128);
+}
+
+int nvfp4_mla_decode_multi_folds(int batch, int q_len, int heads, int max_kv_len, int precision) {
+  g_error[0] = 0;
+  DeviceInfo* d;
+  if (device_info(&d)) return -1;
+  if (precision != NVFP4_MLA_PRECISION_BF16 || batch <= 0 || q_len < 2 || heads <= 0 || heads % 16 != 0 || (long long)q_len * heads > (1 << 16)) return 0;
+  return wants_hm16(q_len * heads, batch, max_kv_len, *d) ? 1 : 0;
+}
+
+int nvfp4_mla_decode_multi(const void* q_nope, const void* q_pe, const uint8_t* ckv_cache, const uint8_t* ckv_sf_cache,
+                           const uint8_t* kpe_cache, int64_t num_pages, int page_size, const int32_t* page_table,
+                           int64_t page_table_stride, const int32_t* kv_lens, int batch, int q_len, int heads, float sm_scale,
+                           float ckv_scale, float kpe_scale, int max_kv_len, int num_splits, int precision, void* out, float* out_f32,
+                           float* lse, void* workspace, int64_t workspace_bytes, void* stream) {
+  g_error[0] = 0;
+  MLA_CHECK(heads > 0 && heads % 16 == 0, "heads must be a multiple of 16, got %d", heads);
+  MLA_CHECK(q_len > 0 && (long long)q_len * heads <= (1 << 16), "q_len must be positive and q_len * heads at most 65536");
+  return decode_impl(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, num_pages, page_size, page_table, page_table_stride, kv_lens,
+                     batch, q_len * heads, sm_scale, ckv_scale, kpe_scale, max_kv_len, num_splits, precision, out, out_f32, lse,
+                     workspace, workspace_bytes, stream, 128, q_len);
 }
 
 // ---- decode without caller-provided scratch -----------------------------------------------------------------------

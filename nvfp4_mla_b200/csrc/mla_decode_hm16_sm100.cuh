@@ -1,5 +1,5 @@
-// Weight-absorbed MLA decode for many query rows per request, 16-bit mode, with the query rows (heads) as the M dimension
-// of both MMAs. The 16-head kernel (mla_decode_vt_sm100.cuh) converts a token once per 16 heads; here one FP16 copy of a
+// Weight-absorbed MLA decode for many query rows per request (heads, or heads x query tokens), 16-bit mode, with the query
+// rows as the M dimension of both MMAs. The 16-head kernel (mla_decode_vt_sm100.cuh) converts a token once per 16 heads; here one FP16 copy of a
 // token serves up to 128 rows:
 //
 //   HBM --L2 prefetch, 16-byte loads--> convert warps' registers --> K/V tile in smem, FP16, [token][channel], 128-byte swizzle
@@ -333,7 +333,15 @@ __device__ __forceinline__ void h16_softmax_role(H16Smem& s, const DecodeParams&
       continue;
     }
     // ---- query: every MMA that read the previous segment's query has completed (the scores of its last tile were consumed)
-    const int hq = h < live_rows ? h : live_rows - 1;  // a dead row of a live quadrant repeats the last one; it is not written out
+    const int hq = h < live_rows ? h : live_rows - 1;
+    // A row sees the tokens up to its own query token: token i of q_len (rows [i, i + 1) * heads / q_len of the request) stops
+    // q_len - 1 - i tokens before the request's end.
+    int row_end = seg.tok_end;
+    if (P.q_len > 1) {
+      const int i = (r0 + hq) / (P.heads / P.q_len), end = P.kv_lens[seg.b] - (P.q_len - 1 - i);
+      row_end = end < row_end ? end : row_end;
+    }
+    // (a dead row of a live quadrant repeats the last live one and is not written out)
     const long long row = (long long)seg.b * P.heads + r0 + hq;
     const uint4* qn = reinterpret_cast<const uint4*>(P.q_nope + row * CKV) + 32 * half;
     const uint4* qp = reinterpret_cast<const uint4*>(P.q_pe + row * KPE);
@@ -410,7 +418,7 @@ __device__ __forceinline__ void h16_softmax_role(H16Smem& s, const DecodeParams&
     for (int t = 0; t < nt; ++t, ++it) {
       const bool ok = ptx::mbar_wait(&s.s_full, it & 1, &s.abort_flag);
       ptx::tc_fence_after_sync();
-      const int nvalid = seg.tok_end - (seg.tok0 + t * kH16Tile) - 32 * half;  // this warp's columns at or beyond it are masked
+      const int nvalid = row_end - (seg.tok0 + t * kH16Tile) - 32 * half;  // this thread's columns at or beyond it are masked
       uint32_t sr[32];
       if (ok) {
         ptx::tmem_ld32(tm_lane + H16Cols::S + 32 * half, sr);

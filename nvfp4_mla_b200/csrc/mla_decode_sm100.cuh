@@ -61,6 +61,7 @@ struct DecodeParams {
   // through linear bulk copies (a box of fewer than 128 bytes cannot be a TMA tile destination): masks 0.
   uint32_t sf_swz_mask, kpe_swz_mask;
   int heads, heads_per_cta;
+  int q_len;       // query tokens per request; `heads` counts the rows of all of them (only the 16-bit heads-as-M kernel takes > 1)
   float sm_scale_log2, ckv_scale, kpe_scale;
   const int2* cta_range;
   const Seg* segs;

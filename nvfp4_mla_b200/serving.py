@@ -8,7 +8,7 @@ checked against the oracle per query position.
 """
 import torch
 
-from . import CKV, KPE, decode, get_batch_indices_positions, quantize_append_paged_mla_kv_cache
+from . import _PRECISIONS, CKV, KPE, _decode, _lib, decode, get_batch_indices_positions, quantize_append_paged_mla_kv_cache
 
 
 def decode_multi_token(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_table, kv_lens, sm_scale,
@@ -19,9 +19,11 @@ def decode_multi_token(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_ta
     cache INCLUDING the ``Q`` new ones, which are its last ``Q`` positions. Query ``i`` attends causally to the first
     ``kv_lens - (Q - 1 - i)`` tokens. Returns ``[batch, Q, heads, 512]`` bfloat16.
 
-    Each query position runs as a request of its own that shares the original's pages (its row of the page table is
-    repeated), so the launch shape stays fixed by ``max_kv_len`` and nothing synchronises; the ``Q`` reads of a request's
-    cache are scheduled next to each other and the later ones are served from L2.
+    With ``precision="bf16"``, enough rows (``Q * heads`` of 64 and more) and enough tokens, all rows of a request share one
+    pass over its cache: one call of the heads-as-M kernel, which cuts each row at its own length. Otherwise each query
+    position runs as a request of its own that shares the original's pages (its row of the page table is repeated); the
+    ``Q`` reads of a request's cache are scheduled next to each other and the later ones are served from L2. Either way the
+    launch shape is fixed by ``max_kv_len`` and nothing synchronises.
     """
     if q_nope.dim() != 4 or q_pe.dim() != 4:
         raise RuntimeError("q_nope must be [batch, Q, heads, 512] and q_pe [batch, Q, heads, 64]")
@@ -30,6 +32,15 @@ def decode_multi_token(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_ta
         raise RuntimeError("q_nope must be [batch, Q, heads, 512] and q_pe [batch, Q, heads, 64]")
     if kv_lens.dim() != 1 or kv_lens.shape[0] != B or kv_lens.dtype != torch.int32:
         raise RuntimeError("kv_lens must be int32 [batch]")
+    if Q > 1 and H > 0 and H % 16 == 0 and ckv_cache.is_cuda and _PRECISIONS.get(precision) == 0:
+        bound = max_kv_len if max_kv_len is not None else int(kv_lens.max()) if B else 0
+        with torch.cuda.device(ckv_cache.device):
+            folds = _lib.load().nvfp4_mla_decode_multi_folds(B, Q, H, int(bound), 0)
+        if folds == 1:
+            out = _decode(q_nope.reshape(B, Q * H, CKV).contiguous(), q_pe.reshape(B, Q * H, KPE).contiguous(), ckv_cache, ckv_sf_cache,
+                          kpe_cache, page_table.contiguous(), kv_lens.contiguous(), sm_scale, ckv_scale, kpe_scale, bound,
+                          num_splits, 0, True, False, q_len=Q)[0]
+            return out.view(B, Q, H, CKV)
     back = torch.arange(Q - 1, -1, -1, dtype=torch.int32, device=kv_lens.device)  # Q-1 .. 0 tokens not yet visible
     lens = (kv_lens[:, None] - back[None, :]).clamp_(min=0).reshape(B * Q).contiguous()
     table = page_table.repeat_interleave(Q, dim=0).contiguous()

@@ -10,6 +10,7 @@ import torch
 
 import mla_oracle as O
 import nvfp4_mla_b200 as mla
+from nvfp4_mla_b200 import _lib, serving
 from nvfp4_mla_b200.testing import SM_SCALE, SyntheticCache
 from util import oracle_reference
 
@@ -80,6 +81,31 @@ def test_wide_range_of_query_magnitudes_and_non_finite_elements():
     c.q_nope[0, 1, 11], c.q_nope[0, 2, 300], c.q_pe[1, 4, 3] = 0.0, 0.0, 0.0
     zeroed, _ = run(c)
     assert np.array_equal(got, zeroed)
+
+
+@pytest.mark.parametrize("q_len,heads", [(2, 32), (4, 16), (5, 16), (3, 64), (2, 128)])
+@pytest.mark.parametrize("num_splits", [0, 2])
+def test_several_query_tokens_in_one_pass(q_len, heads, num_splits):
+    """Requests shorter than q_len, lengths around the tile (a tile that only the last tokens see), rows in two groups."""
+    lens = [6000, 1, 2, 64, 65, 66, 129, 4, 640]
+    c = SyntheticCache(lens, 64, heads, 0.5, 2.0, seed=q_len).to("cuda")
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q_nope = torch.randn(len(lens), q_len, heads, 512, generator=g, device="cuda").bfloat16()
+    q_pe = torch.randn(len(lens), q_len, heads, 64, generator=g, device="cuda").bfloat16()
+    assert _lib.load().nvfp4_mla_decode_multi_folds(len(lens), q_len, heads, max(lens), 0) == 1
+    out = serving.decode_multi_token(q_nope, q_pe, c.ckv_cache, c.ckv_sf_cache, c.kpe_cache, c.page_table, c.kv_lens, SM_SCALE,
+                                     c.ckv_scale, c.kpe_scale, max_kv_len=max(lens), num_splits=num_splits)
+    assert mla.workspace_status() == 0
+    for i in range(q_len):
+        c.q_nope, c.q_pe = q_nope[:, i].contiguous(), q_pe[:, i].contiguous()
+        c.kv_lens_list = [max(n - (q_len - 1 - i), 0) for n in lens]
+        c.kv_lens = torch.tensor(c.kv_lens_list, dtype=torch.int32)
+        want, _ = oracle_reference(c)
+        got = out[:, i].float().cpu().numpy()
+        live = [b for b, n in enumerate(c.kv_lens_list) if n > 0]
+        assert np.abs(got - want).max() <= 2e-2 and O.rel_l2(got[live], want[live]) < 4e-3
+        for b, n in enumerate(c.kv_lens_list):
+            assert n > 0 or (got[b] == 0).all()
 
 
 def test_both_sides_of_the_dispatch_agree():
