@@ -531,8 +531,8 @@ int nvfp4_mla_dequantize(const uint8_t* ckv_cache, const uint8_t* ckv_sf_cache, 
             "ckv_cache must be 4-byte and kpe_cache 2-byte aligned, ckv_out 16-byte and kpe_out 8-byte aligned");
   DeviceInfo* d;
   if (device_info(&d)) return 1;
-  const long long warps_per_block = mla::kDequantThreads / 32;
-  long long blocks = (num_tokens + warps_per_block - 1) / warps_per_block;
+  const long long per_block = mla::kDequantThreads / 32 * mla::kDequantTokens;
+  long long blocks = (num_tokens + per_block - 1) / per_block;
   const long long cap = (long long)d->sm_count * 32;  // grid-stride beyond 32 CTAs per SM
   if (blocks > cap) blocks = cap;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
