@@ -5,13 +5,18 @@
 //   0 where the scale is 0; two codes per byte, low nibble = even channel;
 //   rope: e4m3_rn(kpe / kpe_scale), saturating.
 // Every step is defined as one fp32 IEEE operation in that order, so the bytes are reproducible on a CPU bit for bit.
-// The 512 divisions per token would make the kernel instruction-bound, so the codes are first computed from
-// x * (1 / scale): that product is within 2^-22 (relative) of the correctly rounded quotient, and the code is a
-// monotone step function of the magnitude, so if the products shrunk and grown by 2^-21 get the same code, the
-// quotient gets it too; a value that sits that close to a rounding boundary is settled on its own: an exact tie (which
-// BF16 inputs hit in a few percent of the scale blocks) by one fused multiply-add, anything else by a real division.
+// The 512 divisions per token would make the kernel instruction-bound, so nothing is divided that a product can settle:
+// with the reciprocal of the divisor shrunk and grown by 2^-21, x * r_down and x * r_up enclose the correctly rounded
+// quotient (each product is within 5 * 2^-24 of its ideal value), and the result is a monotone step function of the
+// magnitude, so if both products round to the same code, the quotient does too. A value that sits closer to a rounding
+// boundary is settled on its own: a latent value that ties exactly (BF16 inputs do in a few percent of the scale blocks) by
+// one fused multiply-add, anything else by the real division. The block scale and the rope pair are treated alike; a
+// power-of-two rope scale needs no enclosure, its products are exact.
 //
-// HBM-bound: 1152 bytes in, 352 bytes out per token. One warp per token per trip; lane l owns scale block l
+// 1152 bytes in, 352 bytes out per token, bound by instruction issue (278 warp instructions per token, 69 % of the issue slots):
+// 596415 tokens in 219.6 us, 233.7 with the divisions of the block scale and the rope (138 at the measured copy bandwidth).
+// Thirty-two tokens per warp with one walk through the page tables for all of them was slower (246.7 us).
+// One warp per token per trip; lane l owns scale block l
 // (channels 16l .. 16l+15: two 16-byte loads, one 8-byte store, the warp writes the token's 256 packed bytes as one
 // contiguous run) and rope channels 2l, 2l+1.
 #pragma once
@@ -57,9 +62,21 @@ mla_quantize_append_kernel(const __nv_bfloat16* __restrict__ ckv, const __nv_bfl
                            const int* __restrict__ kv_indptr, int batch, float ckv_scale, float kpe_scale, int* status) {
   const int lane = threadIdx.x & 31;
   constexpr float kDown = 1.f - 0x1p-21f, kUp = 1.f + 0x1p-21f;
+  // reciprocals of the divisors that are the same for every token, as enclosures; divisors near the ends of the fp32 range
+  // (where a product or a reciprocal need not be a normal number) take the divisions
+  auto ordinary = [](float d) { return d > 0x1p-100f && d < 0x1p100f; };
+  const float six = __fmul_rn(6.0f, ckv_scale), r_six = __frcp_rn(six), r_kpe = __frcp_rn(kpe_scale);
+  const bool fast_sf = ordinary(six), fast_kpe = ordinary(kpe_scale);
+  const bool kpe_pow2 = (__float_as_uint(kpe_scale) & 0x007FFFFFu) == 0u;
+  const float six_dn = r_six * kDown, six_up = r_six * kUp;
+  const float kpe_dn = kpe_pow2 ? r_kpe : r_kpe * kDown, kpe_up = kpe_pow2 ? r_kpe : r_kpe * kUp;
   const long long warp0 = (long long)blockIdx.x * (kQuantThreads / 32) + (threadIdx.x >> 5);
   const long long stride = (long long)gridDim.x * (kQuantThreads / 32);
   for (long long t = warp0; t < nnz; t += stride) {
+    // the row itself does not wait for the walk through the page tables
+    const uint4* src = reinterpret_cast<const uint4*>(ckv + t * CKV + 16 * lane);
+    const uint4 w0 = src[0], w1 = src[1];
+    const uint32_t rope = reinterpret_cast<const uint32_t*>(kpe + t * KPE)[lane];
     const int b = batch_indices[t], pos = positions[t];
     bool ok = b >= 0 && b < batch && pos >= 0;
     long long row = 0;
@@ -77,8 +94,6 @@ mla_quantize_append_kernel(const __nv_bfloat16* __restrict__ ckv, const __nv_bfl
       continue;
     }
     // ---- latent block `lane`
-    const uint4* src = reinterpret_cast<const uint4*>(ckv + t * CKV + 16 * lane);
-    const uint4 w0 = src[0], w1 = src[1];
     const uint32_t w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
     float x[16];
     float amax = 0.f;
@@ -87,17 +102,16 @@ mla_quantize_append_kernel(const __nv_bfloat16* __restrict__ ckv, const __nv_bfl
       x[2 * j] = __uint_as_float(w[j] << 16), x[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
       amax = fmaxf(amax, fmaxf(fabsf(x[2 * j]), fabsf(x[2 * j + 1])));
     }
-    const uint32_t sf8 = f32x2_to_e4m3x2_sat(__fdiv_rn(__fdiv_rn(amax, 6.0f), ckv_scale), 0.f) & 0xFFu;
+    const uint32_t sf2 = f32x2_to_e4m3x2_sat(amax * six_dn, amax * six_up);
+    uint32_t sf8 = sf2 & 0xFFu;
+    if (!fast_sf || sf8 != sf2 >> 8) sf8 = f32x2_to_e4m3x2_sat(__fdiv_rn(__fdiv_rn(amax, 6.0f), ckv_scale), 0.f) & 0xFFu;
     const float sf = __fmul_rn(e4m3_value(uint8_t(sf8)), ckv_scale);
     uint32_t lo = 0, hi = 0;
     if (sf > 0.f) {
-      const float r = __frcp_rn(sf), down = kDown, up = kUp;
+      const float r = __frcp_rn(sf), rd = r * kDown, ru = r * kUp;
       float yd[16], yu[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const float q0 = x[j] * r;
-        yd[j] = q0 * down, yu[j] = q0 * up;
-      }
+      for (int j = 0; j < 16; ++j) yd[j] = x[j] * rd, yu[j] = x[j] * ru;
       lo = e2m1x8(reinterpret_cast<const float(&)[8]>(yd[0])), hi = e2m1x8(reinterpret_cast<const float(&)[8]>(yd[8]));
       const uint32_t dlo = lo ^ e2m1x8(reinterpret_cast<const float(&)[8]>(yu[0]));
       const uint32_t dhi = hi ^ e2m1x8(reinterpret_cast<const float(&)[8]>(yu[8]));
@@ -122,9 +136,10 @@ mla_quantize_append_kernel(const __nv_bfloat16* __restrict__ ckv, const __nv_bfl
     *reinterpret_cast<uint2*>(ckv_cache + row * (CKV / 2) + 8 * lane) = make_uint2(lo, hi);
     sf_cache[row * (CKV / 16) + lane] = uint8_t(sf8);
     // ---- rope channels 2 lane, 2 lane + 1
-    const uint32_t r = reinterpret_cast<const uint32_t*>(kpe + t * KPE)[lane];
-    const uint32_t k8 = f32x2_to_e4m3x2_sat(__fdiv_rn(__uint_as_float(r << 16), kpe_scale),
-                                            __fdiv_rn(__uint_as_float(r & 0xFFFF0000u), kpe_scale));
+    const float x0 = __uint_as_float(rope << 16), x1 = __uint_as_float(rope & 0xFFFF0000u);
+    uint32_t k8 = f32x2_to_e4m3x2_sat(x0 * kpe_dn, x1 * kpe_dn);
+    if (!fast_kpe || k8 != f32x2_to_e4m3x2_sat(x0 * kpe_up, x1 * kpe_up))
+      k8 = f32x2_to_e4m3x2_sat(__fdiv_rn(x0, kpe_scale), __fdiv_rn(x1, kpe_scale));
     reinterpret_cast<uint16_t*>(kpe_cache + row * KPE)[lane] = uint16_t(k8);
   }
 }
