@@ -4,6 +4,8 @@ Drop-in for the reference project's ``nvfp4_mla`` package (nvfp4_mla/__init__.py
 ``dequantize`` signatures, defaults, exception types and messages. The work is done by hand-written CUDA kernels in
 ``libnvfp4_mla_b200.so`` behind a C ABI (``include/nvfp4_mla_b200.h``); torch only owns the memory and the stream.
 """
+import functools
+
 import torch
 
 from . import _lib
@@ -52,6 +54,23 @@ def _workspace(device, stream, nbytes):
     return ws
 
 
+@functools.lru_cache(maxsize=4096)
+def _workspace_bytes(device_index, batch, heads, num_splits):
+    """Workspace of a decode call on the current device (``device_index``): a function of the sizes and the GPU alone."""
+    nbytes = _lib.load().nvfp4_mla_decode_workspace_bytes(batch, heads, num_splits)
+    if nbytes < 0:
+        raise RuntimeError(_lib.load().nvfp4_mla_last_error().decode())
+    return nbytes
+
+
+def _on_device(dev, call):
+    """``call()`` with ``dev`` as the current CUDA device (the usual case needs no switch)."""
+    if torch.cuda.current_device() == dev.index:
+        return call()
+    with torch.cuda.device(dev):
+        return call()
+
+
 def _decode(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_table, kv_lens, sm_scale, ckv_scale, kpe_scale,
             max_kv_len, num_splits, precision, want_out, want_partial, partial_into=None, q_len=1):
     # q_len > 1: dimension 1 of the queries holds the heads of q_len query tokens, token by token
@@ -79,30 +98,30 @@ def _decode(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_table, kv_len
         raise RuntimeError("page_size must be a power of two")
     if max_kv_len is None:
         max_kv_len = int(kv_lens.max()) if B else 0  # device sync; pass max_kv_len to avoid it
-    lib = _lib.load()
     dev = ckv_cache.device
-    with torch.cuda.device(dev):
+    if partial_into is not None:
+        o32, lse = partial_into
+        if not (o32.dtype == lse.dtype == torch.float32 and tuple(o32.shape) == (B, H, CKV) and tuple(lse.shape) == (B, H)
+                and o32.is_contiguous() and lse.is_contiguous() and o32.device == dev and lse.device == dev):
+            raise RuntimeError("into must be contiguous float32 ([batch, heads, 512], [batch, heads]) tensors on the cache device")
+    else:
+        o32 = torch.empty(B, H, CKV, dtype=torch.float32, device=dev) if want_partial else None
+        lse = torch.empty(B, H, dtype=torch.float32, device=dev) if want_partial else None
+
+    def launch():
+        lib = _lib.load()
         stream = torch.cuda.current_stream(dev).cuda_stream
-        nbytes = lib.nvfp4_mla_decode_workspace_bytes(B, H, int(num_splits))
-        if nbytes < 0:
-            raise RuntimeError(lib.nvfp4_mla_last_error().decode())
-        ws = _workspace(dev, stream, nbytes)
+        ws = _workspace(dev, stream, _workspace_bytes(dev.index, B, H, int(num_splits)))
         out = torch.empty(B, H, CKV, dtype=torch.bfloat16, device=dev) if want_out else None
-        if partial_into is not None:
-            o32, lse = partial_into
-            if not (o32.dtype == lse.dtype == torch.float32 and tuple(o32.shape) == (B, H, CKV) and tuple(lse.shape) == (B, H)
-                    and o32.is_contiguous() and lse.is_contiguous() and o32.device == dev and lse.device == dev):
-                raise RuntimeError("into must be contiguous float32 ([batch, heads, 512], [batch, heads]) tensors on the cache device")
-        else:
-            o32 = torch.empty(B, H, CKV, dtype=torch.float32, device=dev) if want_partial else None
-            lse = torch.empty(B, H, dtype=torch.float32, device=dev) if want_partial else None
         fn, rows = (lib.nvfp4_mla_decode, (H,)) if q_len == 1 else (lib.nvfp4_mla_decode_multi, (q_len, H // q_len))
         _lib.check(fn(
-            _ptr(q_nope), _ptr(q_pe), _ptr(ckv_cache), _ptr(ckv_sf_cache), _ptr(kpe_cache), ckv_cache.shape[0], ps,
-            _ptr(page_table), page_table.stride(0), _ptr(kv_lens), B, *rows, float(sm_scale), float(ckv_scale),
+            q_nope.data_ptr(), q_pe.data_ptr(), ckv_cache.data_ptr(), ckv_sf_cache.data_ptr(), kpe_cache.data_ptr(), ckv_cache.shape[0], ps,
+            page_table.data_ptr(), page_table.stride(0), kv_lens.data_ptr(), B, *rows, float(sm_scale), float(ckv_scale),
             float(kpe_scale), int(max_kv_len), int(num_splits), int(precision), _ptr(out), _ptr(o32), _ptr(lse),
-            _ptr(ws), ws.numel(), stream))
-    return out, o32, lse
+            ws.data_ptr(), ws.numel(), stream))
+        return out, o32, lse
+
+    return _on_device(dev, launch)
 
 
 def decode(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_table, kv_lens, sm_scale,
@@ -299,12 +318,10 @@ def quantize_append_paged_mla_kv_cache(ckv, kpe, batch_indices, positions, ckv_c
     P, ps = ckv_cache.shape[:2]
     dev = ckv_cache.device
     status = torch.zeros(1, dtype=torch.int32, device=dev) if check else None
-    lib = _lib.load()
-    with torch.cuda.device(dev):
-        _lib.check(lib.nvfp4_mla_quantize_append(
-            _ptr(ckv), _ptr(kpe), _ptr(batch_indices), _ptr(positions), nnz, _ptr(ckv_cache), _ptr(ckv_sf_cache),
-            _ptr(kpe_cache), P, ps, _ptr(kv_indices), _ptr(kv_indptr), kv_indptr.numel() - 1, float(ckv_scale),
-            float(kpe_scale), _ptr(status) if check else None, torch.cuda.current_stream(dev).cuda_stream))
+    _on_device(dev, lambda: _lib.check(_lib.load().nvfp4_mla_quantize_append(
+        _ptr(ckv), _ptr(kpe), _ptr(batch_indices), _ptr(positions), nnz, _ptr(ckv_cache), _ptr(ckv_sf_cache),
+        _ptr(kpe_cache), P, ps, _ptr(kv_indices), _ptr(kv_indptr), kv_indptr.numel() - 1, float(ckv_scale),
+        float(kpe_scale), _ptr(status) if check else None, torch.cuda.current_stream(dev).cuda_stream)))
     if check and int(status.item()) != 0:
         raise RuntimeError("quantize_append: a token named a request, position or page outside the tables")
 

@@ -6,9 +6,10 @@ The reference lists these as what comes next around its kernel (README.md:88, 11
 project): it has none of them, so there is no reference code to mirror; the arithmetic is the decode path's own and is
 checked against the oracle per query position.
 """
+import numpy as np
 import torch
 
-from . import _PRECISIONS, CKV, KPE, _decode, _lib, decode, get_batch_indices_positions, quantize_append_paged_mla_kv_cache
+from . import _PRECISIONS, CKV, KPE, _decode, _lib, decode, quantize_append_paged_mla_kv_cache
 
 
 def decode_multi_token(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_table, kv_lens, sm_scale,
@@ -53,7 +54,8 @@ class PagedLatentCache:
     """A fixed pool of NVFP4 latent-KV pages with per-request page lists: what a serving engine keeps per layer.
 
     Pages are handed out on the host (a free list), the page table and lengths live on the device, and every append
-    goes through the CUDA cache writer. ``max_pages_per_request`` fixes the page-table width, ``max_kv_len`` the decode
+    goes through the CUDA cache writer. What a call has to tell the device (page ids, lengths, token positions) is put
+    together on the host, which knows all of it, and crosses in one copy from pinned memory: no call waits for the GPU. ``max_pages_per_request`` fixes the page-table width, ``max_kv_len`` the decode
     launch shape, so a decode step can be captured in a CUDA graph once the pages of the step have been reserved.
     """
 
@@ -63,12 +65,17 @@ class PagedLatentCache:
         self.ckv_cache = torch.zeros(num_pages, page_size, CKV // 2, dtype=torch.uint8, device=dev)
         self.ckv_sf_cache = torch.zeros(num_pages, page_size, CKV // 16, dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn)
         self.kpe_cache = torch.zeros(num_pages, page_size, KPE, dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn)
-        self.page_table = torch.zeros(max_requests, max_pages_per_request, dtype=torch.int32, device=dev)
-        self.kv_lens = torch.zeros(max_requests, dtype=torch.int32, device=dev)
+        # page table and lengths share one array, so that an append updates both at once
+        self._tables = torch.zeros(max_requests * (max_pages_per_request + 1), dtype=torch.int32, device=dev)
+        self.page_table = self._tables[:max_requests * max_pages_per_request].view(max_requests, max_pages_per_request)
+        self.kv_lens = self._tables[max_requests * max_pages_per_request:]
         self.max_kv_len = max_pages_per_request * page_size
         self._free = list(range(num_pages - 1, -1, -1))
         self._pages = [[] for _ in range(max_requests)]   # host mirror of the page lists
         self._lens = [0] * max_requests                   # host mirror of the lengths
+        # the page table as the writer's page list: request r owns entries [r * width, (r + 1) * width)
+        self._kv_indptr = torch.arange(0, (max_requests + 1) * max_pages_per_request, max(max_pages_per_request, 1),
+                                       dtype=torch.int32, device=dev)
 
     @property
     def free_pages(self):
@@ -78,44 +85,72 @@ class PagedLatentCache:
         """Returns the request's pages to the pool."""
         self._free.extend(reversed(self._pages[request]))
         self._pages[request], self._lens[request] = [], 0
-        self.kv_lens[request] = 0
+        self.kv_lens[request].zero_()
 
     def append(self, requests, ckv, kpe):
         """Appends ``counts[i]`` new tokens to ``requests[i]``: ``requests`` is a list of ``(request, count)`` pairs and
         ``ckv [sum(counts), 512]`` / ``kpe [sum(counts), 64]`` (bfloat16) hold their latent rows in that order."""
-        dev = self.ckv_cache.device
-        new_rows = []
+        if not requests:
+            raise IndexError("append needs at least one request")
+        width, known = self.page_table.shape[1], len(self._lens)
+        slots, values = [], []  # entries of the page table and of the lengths, and what they become
         for r, n in requests:
-            need = -(-(self._lens[r] + n) // self.page_size) - len(self._pages[r])
-            if need > len(self._free) or len(self._pages[r]) + need > self.page_table.shape[1]:
+            pages = self._pages[r]
+            need = -(-(self._lens[r] + n) // self.page_size) - len(pages)
+            if need > len(self._free) or len(pages) + need > width:
                 raise RuntimeError("out of cache pages")
-            for _ in range(need):
-                new_rows.append((r, len(self._pages[r]), self._free.pop()))
-                self._pages[r].append(new_rows[-1][2])
+            if need > 0:
+                at = r % known * width + len(pages)
+                slots += range(at, at + need)
+                pages += self._free[:-need - 1:-1]
+                del self._free[-need:]
+                values += pages[-need:]
             self._lens[r] += n
-        if new_rows:
-            idx = torch.tensor(new_rows, dtype=torch.int64, device=dev)
-            self.page_table[idx[:, 0], idx[:, 1]] = idx[:, 2].int()
-        reqs = [r for r, _ in requests]
-        counts = torch.tensor([0] + [n for _, n in requests], device=dev)
-        nnz = int(counts.sum())
-        lens = torch.tensor([self._lens[r] for r in reqs], dtype=torch.int32, device=dev)
-        self.kv_lens[torch.tensor(reqs, device=dev)] = lens
-        bi, pos = get_batch_indices_positions(counts.cumsum(0).int(), lens, nnz)
-        # the writer addresses pages through (kv_indices, kv_indptr): the rows of the page table of the named requests
-        width = self.page_table.shape[1]
-        kv_indices = self.page_table[torch.tensor(reqs, device=dev)].reshape(-1).contiguous()
-        kv_indptr = (torch.arange(len(reqs) + 1, device=dev) * width).int()
-        quantize_append_paged_mla_kv_cache(ckv, kpe, bi, pos, self.ckv_cache, self.ckv_sf_cache, self.kpe_cache, kv_indices,
-                                           kv_indptr, None, self.ckv_scale, self.kpe_scale)
+        reqs = [r % known for r, _ in requests]
+        lens = [self._lens[r] for r in reqs]
+        slots += [known * width + r for r in reqs]
+        values += lens
+        counts = np.array([n for _, n in requests])
+        nnz, n_slots = int(counts.sum()), len(slots)
+        # position of token j of request i's share: lens[i] - counts[i] + j
+        first = np.cumsum(counts) - counts
+
+        def fill(host):
+            host[:8 * n_slots].view(np.int64)[:] = slots
+            words = host[8 * n_slots:].view(np.int32)
+            words[:n_slots] = values
+            words[n_slots:n_slots + nnz] = np.repeat(reqs, counts)
+            words[n_slots + nnz:] = np.arange(nnz) + np.repeat(lens - counts - first, counts)
+
+        told = self._to_device(12 * n_slots + 8 * nnz, fill)
+        words = told[8 * n_slots:].view(torch.int32)
+        self._tables.index_copy_(0, told[:8 * n_slots].view(torch.int64), words[:n_slots])
+        quantize_append_paged_mla_kv_cache(ckv, kpe, words[n_slots:n_slots + nnz], words[n_slots + nnz:], self.ckv_cache, self.ckv_sf_cache,
+                                           self.kpe_cache, self.page_table.view(-1), self._kv_indptr, None, self.ckv_scale, self.kpe_scale)
+
+    def _to_device(self, nbytes, fill):
+        """A uint8 device copy of ``nbytes`` that ``fill`` writes into a host array, through one copy from pinned memory (the
+        block returns to torch's host allocator, which hands it out again only after the copy has run)."""
+        if torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("a graph cannot capture this call: it would replay today's host data")
+        staged = torch.empty(nbytes, dtype=torch.uint8, pin_memory=True)
+        fill(staged.numpy())
+        return staged.to(self.ckv_cache.device, non_blocking=True)
 
     def decode(self, requests, q_nope, q_pe, sm_scale, w_uv=None, precision="bf16"):
         """One decode step for ``requests`` (a list of request ids): ``q_nope [len(requests), heads, 512]``,
         ``q_pe [len(requests), heads, 64]``. Returns the latent output ``[n, heads, 512]``, or, with
         ``w_uv [heads, 512, v_head_dim]``, the value-space output ``[n, heads, v_head_dim]`` (the absorbed W_UV applied
         after attention)."""
-        idx = torch.tensor(requests, device=self.ckv_cache.device)
-        out = decode(q_nope, q_pe, self.ckv_cache, self.ckv_sf_cache, self.kpe_cache, self.page_table[idx].contiguous(),
-                     self.kv_lens[idx].contiguous(), sm_scale, self.ckv_scale, self.kpe_scale, max_kv_len=self.max_kv_len,
-                     precision=precision)
+        if torch.is_tensor(requests):
+            table, lens = self.page_table[requests.to(self.page_table.device)], self.kv_lens[requests.to(self.page_table.device)]
+        else:
+            ids = np.array(requests, dtype=np.int64)
+            if ids.size and not (-len(self._lens) <= ids.min() and ids.max() < len(self._lens)):
+                raise IndexError("request id out of range")
+            ids %= len(self._lens)
+            idx = self._to_device(ids.nbytes, lambda host: host.__setitem__(slice(None), ids.view(np.uint8))).view(torch.int64)
+            table, lens = self.page_table.index_select(0, idx), self.kv_lens.index_select(0, idx)
+        out = decode(q_nope, q_pe, self.ckv_cache, self.ckv_sf_cache, self.kpe_cache, table, lens, sm_scale, self.ckv_scale,
+                     self.kpe_scale, max_kv_len=self.max_kv_len, precision=precision)
         return out if w_uv is None else torch.einsum("bhc,hcv->bhv", out, w_uv.to(out.dtype))

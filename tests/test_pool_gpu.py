@@ -1,0 +1,55 @@
+"""The paged pool's bookkeeping on the device against its host mirror: page-crossing appends, ragged counts, zero counts, a
+request named twice, release and reuse of pages, and what it refuses."""
+import numpy as np
+import pytest
+import torch
+
+import mla_oracle as O
+from nvfp4_mla_b200 import serving
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("page_size", [1, 16, 64])
+def test_appends_land_where_the_page_table_says(page_size):
+    rng = np.random.default_rng(page_size)
+    pool = serving.PagedLatentCache(700, page_size, 5, 400, 0.5, 2.0)
+    rows = {r: [] for r in range(5)}
+    for step in [[(0, 3), (3, 0), (4, 130)], [(3, 1), (0, 64)], [(2, 65), (1, 1), (0, 1)], "release 0", [(0, 40), (4, 2)]]:
+        if step == "release 0":
+            pool.release(0)
+            rows[0] = []
+            continue
+        n = sum(c for _, c in step)
+        ckv = torch.from_numpy(rng.standard_normal((n, 512), dtype=np.float32)).bfloat16()
+        kpe = torch.from_numpy(rng.standard_normal((n, 64), dtype=np.float32)).bfloat16()
+        at = 0
+        for r, c in step:
+            rows[r] += list(ckv[at:at + c])
+            at += c
+        pool.append(step, ckv.cuda(), kpe.cuda())
+        table, lens, cache = pool.page_table.cpu(), pool.kv_lens.cpu(), pool.ckv_cache.cpu()
+        for r in range(5):
+            assert int(lens[r]) == len(rows[r]) == pool._lens[r]
+            assert table[r, :len(pool._pages[r])].tolist() == pool._pages[r]
+            if rows[r]:
+                t = torch.arange(len(rows[r]))
+                packed, _ = O.quantize_ckv(torch.stack(rows[r]).float().numpy(), 0.5)
+                assert np.array_equal(cache[table[r][t // page_size].long(), t % page_size].numpy(), packed)
+
+
+def test_refusals():
+    pool = serving.PagedLatentCache(4, 16, 2, 3, 0.5, 2.0)
+    z = lambda n: (torch.zeros(n, 512, dtype=torch.bfloat16, device="cuda"), torch.zeros(n, 64, dtype=torch.bfloat16, device="cuda"))
+    with pytest.raises(IndexError):
+        pool.append([], *z(0))
+    with pytest.raises(RuntimeError, match="out of cache pages"):
+        pool.append([(0, 49)], *z(49))
+    with pytest.raises(RuntimeError, match="batch_indices"):
+        pool.append([(1, 3)], *z(4))
+    pool.append([(1, 3)], *z(3))
+    q = torch.zeros(1, 16, 512, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, 16, 64, dtype=torch.bfloat16, device="cuda")
+    for bad in (2, -3):
+        with pytest.raises(IndexError):
+            pool.decode([bad], *q, 0.1)
+    assert torch.equal(pool.decode([1], *q, 0.1), pool.decode(torch.tensor([-1]), *q, 0.1))
