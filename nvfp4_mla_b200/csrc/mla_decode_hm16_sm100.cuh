@@ -260,6 +260,7 @@ __device__ __forceinline__ void h16_qk_role(H16Smem& s, const DecodeParams& P, i
       // the softmax warps have read the scores of tile it - 1; part A of this tile is in place
       if (!__all_sync(~0u, it < 1 || ptx::mbar_wait(&s.s_free, (it - 1) & 1, &s.abort_flag))) return;
       if (!__all_sync(~0u, ptx::mbar_wait(&s.full_a[kb], (it >> 1) & 1, &s.abort_flag))) return;
+      __syncwarp();  // (the issue code's operands live in uniform registers: the warp has to run it as one)
       ptx::tc_fence_after_sync();
       half(cg ^ 1, 0u);
 #pragma unroll
@@ -268,6 +269,7 @@ __device__ __forceinline__ void h16_qk_role(H16Smem& s, const DecodeParams& P, i
       if (leader) ptx::mma_commit(&s.free_a[kb]);
       __syncwarp();
       if (!__all_sync(~0u, ptx::mbar_wait(&s.full_b[kb], (it >> 1) & 1, &s.abort_flag))) return;
+      __syncwarp();
       ptx::tc_fence_after_sync();
       half(cg, 1u);
       if (leader) ptx::mma_commit(&s.s_full);
@@ -286,6 +288,7 @@ __device__ __forceinline__ void h16_pv_role(H16Smem& s, const DecodeParams& P, i
     for (int t = 0; t < nt; ++t, ++it) {
       const uint32_t kb = it & 1;
       if (!__all_sync(~0u, ptx::mbar_wait(&s.p_full, it & 1, &s.abort_flag))) return;
+      __syncwarp();
       ptx::tc_fence_after_sync();
       const uint64_t v_desc = ptx::smem_desc_sw128(ptx::smem_u32(s.kv[kb][4 * cg]), kH16Panel, 1024);
 #pragma unroll

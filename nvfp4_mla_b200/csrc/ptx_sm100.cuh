@@ -325,7 +325,8 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
 }
 // The same two, issued by the one thread of the warp whose `lead` is set, without a branch, and with the operand descriptors
 // as their low words (start address and LBO; a K step or panel is one 32-bit addition) plus a constant high word: fewer
-// registers and instructions per MMA where a warp issues dozens of short ones per tile.
+// registers and instructions per MMA where a warp issues dozens of short ones per tile. The warp has to run them converged (a
+// __syncwarp in front): the operands live in uniform registers, which two diverged halves of a warp would share.
 __device__ __forceinline__ void mma_f16_ss_if(uint32_t lead, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc,
                                               uint32_t accum) {
   asm volatile(
