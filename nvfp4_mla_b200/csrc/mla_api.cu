@@ -1,6 +1,7 @@
 // C ABI of libnvfp4_mla_b200.so: argument validation, the TMA descriptor of the cache, and kernel launches.
 // Declarations and their documentation: include/nvfp4_mla_b200.h.
 #include <climits>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -61,14 +62,22 @@ constexpr int kRawSlotsHm = 4;  // heads-as-M kernel: staging slots of 32 tokens
 // `limit` caps the grouping (a caller with little scratch asks for a narrower one: the partial results of a CTA take
 // 2 KB per head).
 //
-// The 16-bit heads-as-M kernel against the 16-head kernel, us a call: a pair of CTAs takes as long for 48 rows as for 128, so
-// it needs enough heads, and its query load and pipeline are longer, so it needs more than about four 128-token tiles x 16
-// heads per SM: (heads, batch, length) 64,1,1K: 31 against 24 us a call; 128,1,8K: 35 / 33; 64,32,512: 31 / 32; 128,32,512:
-// 40 / 54; 64,128,300: 64 / 76; 64,32 ragged 500..16K: 137 / 171; 128,64,16K: 415 / 833; 128,2,1M: 884 / 1740.
+// The 16-bit heads-as-M kernel against the 16-head kernel. A pair of CTAs takes as long for 48 rows as for 128, so it needs
+// enough heads; a call and a request boundary cost it more, a 128-token tile of many heads less. The choice is between two
+// cost estimates in us, fitted to 59 sizes (64 and 128 heads, 1 to 128 requests, 100 to 160000 tokens):
+//   16-head kernel    : 20 + 2.4 per tile of the fullest CTA + 9 per (request, head group) and CTA
+//   heads-as-M kernel : 42 + 3.6 per tile of the fullest pair + 8.4 per (request, head group) and pair
+// Measured (16-head / heads-as-M), heads, requests, tokens: 64,8,2560: 27 / 42; 128,2,16000: 50 / 56; 128,1,51200: 62 / 54;
+// 64,128,800: 118 / 97; 128,32,1000: 74 / 47; 128,128,625: 146 / 122; 64,32 ragged 500..16000: 172 / 136; 128,64,16384:
+// 833 / 420; 128,2,1M: 1740 / 881.
 constexpr int kHm16MinHeads = 64;
 bool wants_hm16(int heads, int batch, int max_kv_len, const DeviceInfo& d) {
-  const long long tiles = (long long)batch * ((max_kv_len + mla::TILE - 1) / mla::TILE) * (heads / 16);
-  return heads >= kHm16MinHeads && tiles > 4ll * d.sm_count;
+  if (heads < kHm16MinHeads || batch <= 0 || max_kv_len <= 0) return false;
+  const double tiles = double(batch) * ((max_kv_len - 1) / mla::TILE + 1), sms = d.sm_count, pairs = d.sm_count / 2;
+  const int groups16 = heads / 16, groups = (heads + mla::kH16Rows - 1) / mla::kH16Rows;
+  const double by16 = 20. + 2.4 * ceil(tiles * groups16 / sms) + 9. * batch * groups16 / sms;
+  const double as_m = 42. + 3.6 * ceil(tiles * groups / pairs) + 8.4 * batch * groups / pairs;
+  return as_m < by16;
 }
 int hm16_group(int heads) {
   const int groups = (heads + mla::kH16Rows - 1) / mla::kH16Rows;

@@ -42,7 +42,8 @@ def check(c, sm_scale=SM_SCALE, num_splits=0, longest=1 << 20):
 @pytest.mark.parametrize("heads", [64, 80, 112, 128, 144, 192, 256])
 @pytest.mark.parametrize("num_splits", [0, 3])
 def test_head_groups(heads, num_splits):
-    check(SyntheticCache([5000, 513, 64, 1], 64, heads, None, None, seed=heads).to("cuda"), num_splits=num_splits, longest=5000)
+    # (three hundred requests of up to 1500 tokens select the kernel; nearly all of them are three tokens long)
+    check(SyntheticCache([1500, 513, 64, 1] + [3] * 296, 64, heads, None, None, seed=heads).to("cuda"), num_splits=num_splits, longest=1500)
 
 
 @pytest.mark.parametrize("page_size", [1, 2, 8, 16, 32, 64, 256])
@@ -87,7 +88,7 @@ def test_wide_range_of_query_magnitudes_and_non_finite_elements():
 @pytest.mark.parametrize("num_splits", [0, 2])
 def test_several_query_tokens_in_one_pass(q_len, heads, num_splits):
     """Requests shorter than q_len, lengths around the tile (a tile that only the last tokens see), rows in two groups."""
-    lens = [6000, 1, 2, 64, 65, 66, 129, 4, 640]
+    lens = [1500, 1, 2, 64, 65, 66, 129, 4, 640] + [7] * 191
     c = SyntheticCache(lens, 64, heads, 0.5, 2.0, seed=q_len).to("cuda")
     g = torch.Generator(device="cuda").manual_seed(1)
     q_nope = torch.randn(len(lens), q_len, heads, 512, generator=g, device="cuda").bfloat16()
@@ -109,11 +110,11 @@ def test_several_query_tokens_in_one_pass(q_len, heads, num_splits):
 
 
 def test_both_sides_of_the_dispatch_agree():
-    """64 heads, ten requests: a bound of 14 tiles per request is the last one of the 16-head kernel on 148 SMs, 15 the first of
-    this one."""
+    """The bound of the lengths chooses the kernel: 512 tokens the 16-head one, 2^20 this one."""
     c = SyntheticCache([400] * 10, 64, 64, None, None, seed=8).to("cuda")
-    few, few_lse = run(c, longest=14 * 128)
-    many, many_lse = run(c, longest=15 * 128)
+    few, few_lse = run(c, longest=512)
+    many, many_lse = run(c, longest=1 << 20)
+    assert not np.array_equal(few, many)  # (they round differently: it is two kernels)
     assert O.rel_l2(few, many) < 4e-3 and np.abs(few_lse - many_lse).max() <= 1e-3
 
 
