@@ -295,16 +295,8 @@ def get_batch_indices_positions(append_indptr, seq_lens, nnz):
     return bi.to(torch.int32), pos.to(torch.int32)
 
 
-def quantize_append_paged_mla_kv_cache(ckv, kpe, batch_indices, positions, ckv_cache, ckv_sf_cache, kpe_cache,
-                                       kv_indices, kv_indptr, kv_last_page_len=None, ckv_scale=1.0, kpe_scale=1.0,
-                                       check=False):
-    """Quantises new tokens to NVFP4 / E4M3 and writes them into the paged cache, in place.
-
-    Same arguments as FlashInfer's ``nvfp4_quantize_append_paged_mla_kv_cache``, the writer the reference uses
-    (``nvfp4_mla/testing.py:51-53``): ``ckv [nnz, 512]`` and ``kpe [nnz, 64]`` bfloat16, ``batch_indices`` /
-    ``positions`` ``[nnz]`` int32, the three cache tensors, the page list ``kv_indices`` with ``kv_indptr [B + 1]``;
-    ``kv_last_page_len`` is accepted and not needed. ``check=True`` synchronises and raises if a token pointed
-    outside the tables (such tokens are skipped)."""
+def _check_append(ckv, kpe, batch_indices, positions, ckv_cache, ckv_sf_cache, kpe_cache, kv_indices, kv_indptr):
+    """What the cache writer refuses; returns the number of rows."""
     _check_cache(ckv_cache, ckv_sf_cache, kpe_cache)
     nnz = ckv.shape[0]
     if ckv.dtype != torch.bfloat16 or kpe.dtype != torch.bfloat16:
@@ -315,6 +307,20 @@ def quantize_append_paged_mla_kv_cache(ckv, kpe, batch_indices, positions, ckv_c
                        ("kv_indptr", kv_indptr, None)):
         if t.dtype != torch.int32 or t.dim() != 1 or not t.is_contiguous() or (n is not None and t.numel() != n):
             raise RuntimeError(f"{name} must be a contiguous 1-D int32 tensor" + (f" of {n} elements" if n is not None else ""))
+    return nnz
+
+
+def quantize_append_paged_mla_kv_cache(ckv, kpe, batch_indices, positions, ckv_cache, ckv_sf_cache, kpe_cache,
+                                       kv_indices, kv_indptr, kv_last_page_len=None, ckv_scale=1.0, kpe_scale=1.0,
+                                       check=False):
+    """Quantises new tokens to NVFP4 / E4M3 and writes them into the paged cache, in place.
+
+    Same arguments as FlashInfer's ``nvfp4_quantize_append_paged_mla_kv_cache``, the writer the reference uses
+    (``nvfp4_mla/testing.py:51-53``): ``ckv [nnz, 512]`` and ``kpe [nnz, 64]`` bfloat16, ``batch_indices`` /
+    ``positions`` ``[nnz]`` int32, the three cache tensors, the page list ``kv_indices`` with ``kv_indptr [B + 1]``;
+    ``kv_last_page_len`` is accepted and not needed. ``check=True`` synchronises and raises if a token pointed
+    outside the tables (such tokens are skipped)."""
+    nnz = _check_append(ckv, kpe, batch_indices, positions, ckv_cache, ckv_sf_cache, kpe_cache, kv_indices, kv_indptr)
     P, ps = ckv_cache.shape[:2]
     dev = ckv_cache.device
     status = torch.zeros(1, dtype=torch.int32, device=dev) if check else None

@@ -6,10 +6,12 @@ The reference lists these as what comes next around its kernel (README.md:88, 11
 project): it has none of them, so there is no reference code to mirror; the arithmetic is the decode path's own and is
 checked against the oracle per query position.
 """
+import operator
+
 import numpy as np
 import torch
 
-from . import _PRECISIONS, CKV, KPE, _decode, _lib, decode, quantize_append_paged_mla_kv_cache
+from . import _PRECISIONS, CKV, KPE, _check_append, _decode, _lib, decode, quantize_append_paged_mla_kv_cache
 
 
 def decode_multi_token(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_table, kv_lens, sm_scale,
@@ -89,30 +91,38 @@ class PagedLatentCache:
 
     def append(self, requests, ckv, kpe):
         """Appends ``counts[i]`` new tokens to ``requests[i]``: ``requests`` is a list of ``(request, count)`` pairs and
-        ``ckv [sum(counts), 512]`` / ``kpe [sum(counts), 64]`` (bfloat16) hold their latent rows in that order."""
+        ``ckv [sum(counts), 512]`` / ``kpe [sum(counts), 64]`` (bfloat16) hold their latent rows in that order.
+        Whatever refuses the call does so before the pool changes."""
         if not requests:
             raise IndexError("append needs at least one request")
         width, known = self.page_table.shape[1], len(self._lens)
         slots, values = [], []  # entries of the page table and of the lengths, and what they become
+        reqs, counts = [], []
+        grown, taken = {}, 0  # per request: [length, new pages]; pages taken from the end of the free list
         for r, n in requests:
-            pages = self._pages[r]
-            need = -(-(self._lens[r] + n) // self.page_size) - len(pages)
-            if need > len(self._free) or len(pages) + need > width:
+            r, n = range(known)[r], operator.index(n)  # (a negative id counts from the end)
+            if n < 0:
+                raise ValueError("counts must not be negative")
+            to = grown.setdefault(r, [self._lens[r], []])
+            held = len(self._pages[r]) + len(to[1])
+            need = -(-(to[0] + n) // self.page_size) - held
+            if need > len(self._free) - taken or held + need > width:
                 raise RuntimeError("out of cache pages")
             if need > 0:
-                at = r % known * width + len(pages)
+                at = r * width + held
                 slots += range(at, at + need)
-                pages += self._free[:-need - 1:-1]
-                del self._free[-need:]
-                values += pages[-need:]
-            self._lens[r] += n
-        reqs = [r % known for r, _ in requests]
-        lens = [self._lens[r] for r in reqs]
-        slots += [known * width + r for r in reqs]
-        values += lens
-        counts = np.array([n for _, n in requests])
+                fresh = self._free[-taken - 1:-taken - need - 1:-1]
+                values += fresh
+                to[1] += fresh
+                taken += need
+            to[0] += n
+            reqs.append(r)
+            counts.append(n)
+        slots += [known * width + r for r in grown]
+        values += [end for end, _ in grown.values()]
+        ends, counts = [grown[r][0] for r in reqs], np.array(counts)
         nnz, n_slots = int(counts.sum()), len(slots)
-        # position of token j of request i's share: lens[i] - counts[i] + j
+        # position of token j of request i's share: ends[i] - counts[i] + j
         first = np.cumsum(counts) - counts
 
         def fill(host):
@@ -120,13 +130,20 @@ class PagedLatentCache:
             words = host[8 * n_slots:].view(np.int32)
             words[:n_slots] = values
             words[n_slots:n_slots + nnz] = np.repeat(reqs, counts)
-            words[n_slots + nnz:] = np.arange(nnz) + np.repeat(lens - counts - first, counts)
+            words[n_slots + nnz:] = np.arange(nnz) + np.repeat(ends - counts - first, counts)
 
         told = self._to_device(12 * n_slots + 8 * nnz, fill)
         words = told[8 * n_slots:].view(torch.int32)
+        write = (ckv, kpe, words[n_slots:n_slots + nnz], words[n_slots + nnz:], self.ckv_cache, self.ckv_sf_cache, self.kpe_cache,
+                 self.page_table.view(-1), self._kv_indptr)
+        if _check_append(*write) and (ckv.data_ptr() % 16 or kpe.data_ptr() % 4):
+            raise RuntimeError("ckv must be 16-byte and kpe 4-byte aligned")
         self._tables.index_copy_(0, told[:8 * n_slots].view(torch.int64), words[:n_slots])
-        quantize_append_paged_mla_kv_cache(ckv, kpe, words[n_slots:n_slots + nnz], words[n_slots + nnz:], self.ckv_cache, self.ckv_sf_cache,
-                                           self.kpe_cache, self.page_table.view(-1), self._kv_indptr, None, self.ckv_scale, self.kpe_scale)
+        quantize_append_paged_mla_kv_cache(*write, None, self.ckv_scale, self.kpe_scale)
+        del self._free[len(self._free) - taken:]
+        for r, (end, fresh) in grown.items():
+            self._lens[r] = end
+            self._pages[r] += fresh
 
     def _to_device(self, nbytes, fill):
         """A uint8 device copy of ``nbytes`` that ``fill`` writes into a host array, through one copy from pinned memory (the

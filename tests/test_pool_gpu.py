@@ -53,3 +53,47 @@ def test_refusals():
         with pytest.raises(IndexError):
             pool.decode([bad], *q, 0.1)
     assert torch.equal(pool.decode([1], *q, 0.1), pool.decode(torch.tensor([-1]), *q, 0.1))
+
+
+def state(pool):
+    return (list(pool._free), [list(p) for p in pool._pages], list(pool._lens), pool.page_table.cpu().tolist(), pool.kv_lens.cpu().tolist())
+
+
+@pytest.mark.parametrize("why", ["pages", "width", "id", "count", "rows", "dtype", "alignment", "capture"])
+def test_a_refused_append_leaves_the_pool_unchanged(why):
+    """Also where an earlier request of the same call could have been served: nothing of it may stay behind on the host, whose
+    next append would tell the device only what it believes to be new."""
+    pool = serving.PagedLatentCache(7, 16, 3, 4, 0.5, 2.0)
+    rows = lambda n, dtype=torch.bfloat16: (torch.zeros(n, 512, dtype=dtype, device="cuda"), torch.zeros(n, 64, dtype=dtype, device="cuda"))
+    pool.append([(2, 20)], *rows(20))
+    before = state(pool)
+    requests, given, error = [(0, 17), (1, 33)], rows(50), RuntimeError
+    if why == "pages":
+        requests, given = [(0, 33), (1, 33)], rows(66)
+    elif why == "width":
+        requests, given = [(0, 17), (2, 45)], rows(62)
+    elif why == "id":
+        requests, given, error = [(0, 17), (3, 1)], rows(18), IndexError
+    elif why == "count":
+        requests, given, error = [(0, 17), (1, -1)], rows(16), ValueError
+    elif why == "rows":
+        requests, given = [(0, 17), (1, 5)], rows(21)
+    elif why == "dtype":
+        requests, given = [(0, 17), (1, 5)], rows(22, torch.float32)
+    elif why == "alignment":
+        requests, given = [(0, 17), (1, 5)], (torch.zeros(22 * 512 + 4, dtype=torch.bfloat16, device="cuda")[4:].view(22, 512), rows(22)[1])
+    else:
+        requests, given = [(0, 17), (1, 5)], rows(22)
+    torch.cuda.synchronize()
+    if why == "capture":
+        with pytest.raises(error), torch.cuda.graph(torch.cuda.CUDAGraph()):
+            pool.append(requests, *given)
+    else:
+        with pytest.raises(error):
+            pool.append(requests, *given)
+    assert state(pool) == before
+    pool.append([(0, 17), (1, 5)], *rows(22))  # what fits is served as if nothing had happened
+    assert pool._lens == [17, 5, 20] == pool.kv_lens.tolist() and pool.free_pages == 2
+    for r in range(3):
+        assert pool.page_table[r, :len(pool._pages[r])].tolist() == pool._pages[r]
+    assert len(sum(pool._pages, [])) == len(set(sum(pool._pages, []))) == 5
