@@ -91,13 +91,13 @@ class PagedLatentCache:
 
     def append(self, requests, ckv, kpe):
         """Appends ``counts[i]`` new tokens to ``requests[i]``: ``requests`` is a list of ``(request, count)`` pairs and
-        ``ckv [sum(counts), 512]`` / ``kpe [sum(counts), 64]`` (bfloat16) hold their latent rows in that order.
-        Whatever refuses the call does so before the pool changes."""
+        ``ckv [sum(counts), 512]`` / ``kpe [sum(counts), 64]`` (bfloat16) hold their latent rows in that order. A request may be
+        named more than once: its shares follow each other. Whatever refuses the call does so before the pool changes."""
         if not requests:
             raise IndexError("append needs at least one request")
         width, known = self.page_table.shape[1], len(self._lens)
         slots, values = [], []  # entries of the page table and of the lengths, and what they become
-        reqs, counts = [], []
+        reqs, counts, ends = [], [], []  # per entry of the call: request, tokens, the request's length after it
         grown, taken = {}, 0  # per request: [length, new pages]; pages taken from the end of the free list
         for r, n in requests:
             r, n = range(known)[r], operator.index(n)  # (a negative id counts from the end)
@@ -118,11 +118,12 @@ class PagedLatentCache:
             to[0] += n
             reqs.append(r)
             counts.append(n)
+            ends.append(to[0])
         slots += [known * width + r for r in grown]
         values += [end for end, _ in grown.values()]
-        ends, counts = [grown[r][0] for r in reqs], np.array(counts)
+        counts = np.array(counts)
         nnz, n_slots = int(counts.sum()), len(slots)
-        # position of token j of request i's share: ends[i] - counts[i] + j
+        # position of token j of entry i: ends[i] - counts[i] + j
         first = np.cumsum(counts) - counts
 
         def fill(host):

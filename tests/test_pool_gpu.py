@@ -55,6 +55,25 @@ def test_refusals():
     assert torch.equal(pool.decode([1], *q, 0.1), pool.decode(torch.tensor([-1]), *q, 0.1))
 
 
+def test_a_request_named_twice_gets_its_shares_one_after_the_other():
+    """The pool's bytes, tables and lengths equal those of a pool that appended the shares in calls of their own."""
+    g = torch.Generator(device="cuda").manual_seed(7)
+    steps = [[(0, 3), (0, 2)], [(1, 20), (0, 14), (1, 1), (0, 30)], [(-3, 1), (0, 0), (0, 2)]]
+    pools = [serving.PagedLatentCache(20, 16, 3, 8, 0.5, 2.0) for _ in range(2)]
+    for step in steps:
+        n = sum(c for _, c in step)
+        ckv, kpe = torch.randn(n, 512, generator=g, device="cuda").bfloat16(), torch.randn(n, 64, generator=g, device="cuda").bfloat16()
+        pools[0].append(step, ckv, kpe)
+        at = 0
+        for r, c in step:
+            pools[1].append([(r, c)], ckv[at:at + c], kpe[at:at + c])
+            at += c
+    assert state(pools[0]) == state(pools[1]) and pools[0]._lens == [52, 21, 0]
+    for name in ("ckv_cache", "ckv_sf_cache", "kpe_cache"):
+        a, b = (getattr(p, name).view(torch.uint8) for p in pools)
+        assert torch.equal(a, b) and int(a.count_nonzero())
+
+
 def state(pool):
     return (list(pool._free), [list(p) for p in pool._pages], list(pool._lens), pool.page_table.cpu().tolist(), pool.kv_lens.cpu().tolist())
 
