@@ -163,12 +163,17 @@ class PagedLatentCache:
         if torch.is_tensor(requests):
             table, lens = self.page_table[requests.to(self.page_table.device)], self.kv_lens[requests.to(self.page_table.device)]
         else:
-            ids = np.array(requests, dtype=np.int64)
-            if ids.size and not (-len(self._lens) <= ids.min() and ids.max() < len(self._lens)):
-                raise IndexError("request id out of range")
-            ids %= len(self._lens)
-            idx = self._to_device(ids.nbytes, lambda host: host.__setitem__(slice(None), ids.view(np.uint8))).view(torch.int64)
-            table, lens = self.page_table.index_select(0, idx), self.kv_lens.index_select(0, idx)
+            ids = torch.tensor(requests)
+            if ids.dim() == 1 and ids.numel() and ids.dtype in (torch.int64, torch.int32):
+                ids = ids.numpy().astype(np.int64)
+                if not (-len(self._lens) <= ids.min() and ids.max() < len(self._lens)):
+                    raise IndexError("request id out of range")
+                ids %= len(self._lens)
+                idx = self._to_device(ids.nbytes, lambda host: host.__setitem__(slice(None), ids.view(np.uint8))).view(torch.int64)
+                table, lens = self.page_table.index_select(0, idx), self.kv_lens.index_select(0, idx)
+            else:  # a mask over all requests; what is neither ids nor a mask is refused by the indexing
+                idx = ids.to(self.page_table.device)
+                table, lens = self.page_table[idx].contiguous(), self.kv_lens[idx].contiguous()
         out = decode(q_nope, q_pe, self.ckv_cache, self.ckv_sf_cache, self.kpe_cache, table, lens, sm_scale, self.ckv_scale,
                      self.kpe_scale, max_kv_len=self.max_kv_len, precision=precision)
         return out if w_uv is None else torch.einsum("bhc,hcv->bhv", out, w_uv.to(out.dtype))

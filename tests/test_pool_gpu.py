@@ -116,3 +116,19 @@ def test_a_refused_append_leaves_the_pool_unchanged(why):
     for r in range(3):
         assert pool.page_table[r, :len(pool._pages[r])].tolist() == pool._pages[r]
     assert len(sum(pool._pages, [])) == len(set(sum(pool._pages, []))) == 5
+
+
+def test_forms_of_request_ids():
+    """Whole numbers in any container, or a mask over all requests; anything else is refused and not read as a number."""
+    pool = serving.PagedLatentCache(8, 16, 2, 3, 0.5, 2.0)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    r = lambda *shape: torch.randn(*shape, generator=g, device="cuda").bfloat16()
+    pool.append([(0, 5), (1, 20)], r(25, 512), r(25, 64))
+    q = r(1, 16, 512), r(1, 16, 64)
+    want = pool.decode([1], *q, 0.1)
+    for ids in ((1,), np.array([1]), np.array([1], dtype=np.int32), [False, True], np.array([False, True]), [torch.tensor(1, device="cuda")],
+                torch.tensor([1]), torch.tensor([1], device="cuda"), torch.tensor([False, True])):
+        assert torch.equal(pool.decode(ids, *q, 0.1), want), ids
+    for ids in ([1.7], [1.0], [], np.array([1.0])):
+        with pytest.raises(IndexError):
+            pool.decode(ids, *q, 0.1)
