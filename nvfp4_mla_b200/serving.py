@@ -26,7 +26,7 @@ def decode_multi_token(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_ta
     pass over its cache: one call of the heads-as-M kernel, which cuts each row at its own length. Otherwise each query
     position runs as a request of its own that shares the original's pages (its row of the page table is repeated); the
     ``Q`` reads of a request's cache are scheduled next to each other and the later ones are served from L2. Either way the
-    launch shape is fixed by ``max_kv_len`` and nothing synchronises.
+    launch shape is fixed by ``max_kv_len``, and nothing synchronises if it is given (one read of the lengths if not).
     """
     if q_nope.dim() != 4 or q_pe.dim() != 4:
         raise RuntimeError("q_nope must be [batch, Q, heads, 512] and q_pe [batch, Q, heads, 64]")
@@ -36,12 +36,13 @@ def decode_multi_token(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_ta
     if kv_lens.dim() != 1 or kv_lens.shape[0] != B or kv_lens.dtype != torch.int32:
         raise RuntimeError("kv_lens must be int32 [batch]")
     if Q > 1 and H > 0 and H % 16 == 0 and ckv_cache.is_cuda and _PRECISIONS.get(precision) == 0:
-        bound = max_kv_len if max_kv_len is not None else int(kv_lens.max()) if B else 0
+        if max_kv_len is None:
+            max_kv_len = int(kv_lens.max()) if B else 0  # device sync; the lengths below are not longer
         with torch.cuda.device(ckv_cache.device):
-            folds = _lib.load().nvfp4_mla_decode_multi_folds(B, Q, H, int(bound), 0)
+            folds = _lib.load().nvfp4_mla_decode_multi_folds(B, Q, H, int(max_kv_len), 0)
         if folds == 1:
             out = _decode(q_nope.reshape(B, Q * H, CKV).contiguous(), q_pe.reshape(B, Q * H, KPE).contiguous(), ckv_cache, ckv_sf_cache,
-                          kpe_cache, page_table.contiguous(), kv_lens.contiguous(), sm_scale, ckv_scale, kpe_scale, bound,
+                          kpe_cache, page_table.contiguous(), kv_lens.contiguous(), sm_scale, ckv_scale, kpe_scale, max_kv_len,
                           num_splits, 0, True, False, q_len=Q)[0]
             return out.view(B, Q, H, CKV)
     back = torch.arange(Q - 1, -1, -1, dtype=torch.int32, device=kv_lens.device)  # Q-1 .. 0 tokens not yet visible

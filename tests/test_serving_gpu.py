@@ -1,5 +1,7 @@
 """GPU tests of the callers around the decode path: multi-token (MTP / speculative verify) decode and the paged
 latent-KV pool (append through the CUDA writer, decode, W_UV). Checked against the numpy oracle per query position."""
+import warnings
+
 import numpy as np
 import pytest
 import torch
@@ -37,6 +39,26 @@ def test_multi_token_decode_matches_oracle_per_position(precision, tol):
             if L == 0:
                 assert (got[b] == 0).all()
     assert mla.workspace_status() == 0
+
+
+@pytest.mark.parametrize("kv_len,folds", [(300, 0), (40000, 1)])
+def test_multi_token_decode_reads_the_lengths_once(kv_len, folds):
+    """Without ``max_kv_len`` the call waits for the device once, whichever way it goes, and not at all with it."""
+    c = SyntheticCache([kv_len] * 2 + [7] * 14, 64, 16, 0.5, 2.0, seed=1, device="cuda")
+    q_nope, q_pe = (c.q_nope[:, None].expand(-1, 4, -1, -1).contiguous(), c.q_pe[:, None].expand(-1, 4, -1, -1).contiguous())
+    assert mla._lib.load().nvfp4_mla_decode_multi_folds(16, 4, 16, kv_len, 0) == folds
+    args = (q_nope, q_pe, c.ckv_cache, c.ckv_sf_cache, c.kpe_cache, c.page_table, c.kv_lens, SM_SCALE, c.ckv_scale, c.kpe_scale)
+    want = serving.decode_multi_token(*args, max_kv_len=kv_len)
+    for given, syncs in ((kv_len, 0), (None, 1)):
+        torch.cuda.set_sync_debug_mode("warn")
+        try:
+            with warnings.catch_warnings(record=True) as seen:
+                warnings.simplefilter("always")
+                out = serving.decode_multi_token(*args, max_kv_len=given)
+        finally:
+            torch.cuda.set_sync_debug_mode("default")
+        assert len([w for w in seen if "synchron" in str(w.message)]) == syncs
+        assert torch.equal(out, want)
 
 
 def test_pool_append_decode_loop():
