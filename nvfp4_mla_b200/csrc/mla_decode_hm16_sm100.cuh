@@ -405,6 +405,7 @@ __device__ __forceinline__ void h16_softmax_role(H16Smem& s, const DecodeParams&
     float down = 1.f;  // what the scores are to be multiplied with
     const bool ordinary = amax >= 0x1p-8f && amax <= 0x1p14f;
     if (!__all_sync(~0u, ordinary)) {  // (both warps of the pair see the same maxima)
+      ptx::tmem_wait_st();             // the first pass's stores go to the same columns: they have to land first
       int e = int(__float_as_uint(amax) >> 23) - 127 - 14;
       e = ordinary ? 0 : e < -94 ? -94 : e > 112 ? 112 : e;
       load_query(sign * __uint_as_float(uint32_t(127 - e) << 23));

@@ -127,3 +127,18 @@ def test_page_ids_are_range_checked(page_size):
     out = mla.decode(*args, max_kv_len=1 << 20)
     assert mla.workspace_status(clear=True) == 3
     assert np.array_equal(out[0].float().cpu().numpy(), good[0]) and torch.isfinite(out.float()).all()
+
+
+@pytest.mark.parametrize("power", [-30, -9, 12, 40])
+def test_query_loaded_a_second_time_replaces_the_first(power):
+    """Rows whose magnitude FP16 cannot hold as they are go through the query load twice, into the same places. A power of two in
+    all queries, taken out again by the softmax scale, changes no bit of the result: the query's elements and their products with the
+    ratio of the two scales (a power of two) are exact in either form."""
+    c = SyntheticCache([1, 130, 7, 64] * 80, 64, 128, 0.5, 2.0, seed=6).to("cuda")
+    c.q_nope, c.q_pe = (c.q_nope * 16).round() / 16, (c.q_pe * 16).round() / 16
+    want, want_lse = run(c)
+    c.q_nope *= 2.0 ** power
+    c.q_pe *= 2.0 ** power
+    for _ in range(5):
+        got, lse = run(c, SM_SCALE * 2.0 ** -power)
+        assert np.array_equal(got, want) and np.array_equal(lse, want_lse)
