@@ -7,8 +7,9 @@
 //                                               B = the K/V tile read K-major, N = 64 tokens
 //   PV   : O[row, chan] += P[row, token] . V    A = P (FP16) from tensor memory, written there by the softmax threads,
 //                                               B = the same K/V tile read MN-major, N = 256 channels, K = 16 tokens
-// Both K and V are exact in FP16 (e2m1 x e4m3 has six significant bits), Q is exact after a power-of-two scaling of the
-// row (a BF16 has eight), the accumulators are fp32.
+// Both K and V are exact in FP16 (e2m1 x e4m3 has six significant bits). The latent part of Q (a BF16 has eight) is
+// held times a power of two per row: exact, but for elements so small that they are off by up to 2^-25 of the row's maximum. Its
+// rope part is multiplied with kpe_scale / ckv_scale and rounded to FP16. The accumulators are fp32.
 //
 // O for 128 rows x 512 channels would need all 512 tensor-memory columns, so a PAIR of CTAs shares a request: both compute
 // the full scores, CTA `cg` accumulates channels [256 cg, 256 cg + 256). The pair is one unit of the schedule and writes one
@@ -394,24 +395,27 @@ __device__ __forceinline__ void h16_softmax_role(H16Smem& s, const DecodeParams&
       }
       return fmaxf(__uint_as_float(max(m2 << 16, m2 & 0xFFFF0000u)), __uint_as_float(max(m2p << 16, m2p & 0xFFFF0000u)) * ratio);
     };
-    // The sign of the softmax scale goes into Q, so that a larger accumulator is always a larger score. FP16 holds the BF16
-    // elements of an ordinary row as they are (exactly from 2^-14 up, to 2^-24 below: 2^-16 of the row's maximum at worst): one
-    // pass over it. A row whose maximum lies outside [2^-8, 2^14] is loaded again times a power of two that puts its maximum
-    // into [2^14, 2^15); the tensor-memory stores are warp-wide, so the pair of warps decides together.
+    // The sign of the softmax scale goes into Q, so that a larger accumulator is always a larger score. The row is held times a power
+    // of two, which the score's scale takes out again. Ordinary rows (maximum in [2^-8, 2^7]) are loaded in one pass, times 2^8:
+    // their elements are exact from 2^-25 up and off by at most 2^-33 below, 2^-25 of the row's maximum (times 1, elements of
+    // 2^-18 that meet large latent values had eight bits of error left). Any other row is loaded again times the power that puts its
+    // maximum into [2^14, 2^15): exact from 2^-31 of the maximum up. The rope elements are products with `ratio`, rounded to FP16's
+    // eleven bits. The tensor-memory stores are warp-wide, so the pair of warps decides together.
+    constexpr int kUp = 8;
     const float sign = P.sm_scale_log2 < 0.f ? -1.f : 1.f;
-    s.xch[half][h] = load_query(sign);
+    s.xch[half][h] = load_query(sign * float(1 << kUp));
     ptx::bar_sync(pair_bar, 64);
     const float amax = fmaxf(s.xch[0][h], s.xch[1][h]);
-    float down = 1.f;  // what the scores are to be multiplied with
-    const bool ordinary = amax >= 0x1p-8f && amax <= 0x1p14f;
+    const bool ordinary = amax >= 0x1p-8f && amax <= 0x1p7f;
+    int e = -kUp;  // the row is held times 2^-e
     if (!__all_sync(~0u, ordinary)) {  // (both warps of the pair see the same maxima)
       ptx::tmem_wait_st();             // the first pass's stores go to the same columns: they have to land first
-      int e = int(__float_as_uint(amax) >> 23) - 127 - 14;
-      e = ordinary ? 0 : e < -94 ? -94 : e > 112 ? 112 : e;
+      e = int(__float_as_uint(amax) >> 23) - 127 - 14;
+      e = ordinary ? -kUp : e < -94 ? -94 : e > 112 ? 112 : e;
       load_query(sign * __uint_as_float(uint32_t(127 - e) << 23));
-      down = __uint_as_float(uint32_t(127 + e) << 23);
     }
-    const float qa = fmaxf(fabsf(P.sm_scale_log2) * P.ckv_scale * down, 1e-37f);
+    // (never 0: a masked score is -inf and must stay so)
+    const float qa = fmaxf(fabsf(P.sm_scale_log2) * P.ckv_scale * __uint_as_float(uint32_t(127 + e) << 23), 0x1p-149f);
     if (half) ptx::fence_proxy_async_smem();
     ptx::tmem_wait_st();
     ptx::tc_fence_before_sync();

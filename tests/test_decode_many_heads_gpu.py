@@ -142,3 +142,20 @@ def test_query_loaded_a_second_time_replaces_the_first(power):
     for _ in range(5):
         got, lse = run(c, SM_SCALE * 2.0 ** -power)
         assert np.array_equal(got, want) and np.array_equal(lse, want_lse)
+
+
+@pytest.mark.parametrize("top", [2.0 ** -8, 2.0 ** -2, 2.0 ** 6])
+def test_small_query_elements_against_large_latents(top):
+    """Half of the channels hold query elements 2^11 below the row's maximum, but meet latent values 2^17 above the others': they
+    decide the scores (standard deviation about 3). Bound: rel-L2 < 4e-3 as elsewhere (the BF16 result alone is 1.7e-3); an error
+    of 2^-25 of the row's maximum per element moves a score by less than 2^-13."""
+    c = SyntheticCache([100, 64, 33] * 100, 64, 64, 4.0 / top, 1.0, seed=12).to("cuda")
+    c.ckv_cache.random_(0, 256, generator=torch.Generator(device="cuda").manual_seed(2))  # all codes alike
+    sf = c.ckv_sf_cache.view(torch.uint8)
+    sf[..., :16], sf[..., 16:] = 0x7E, 0x01  # 448 and 2^-9
+    c.q_nope[..., :256] *= top * 2.0 ** -11
+    c.q_nope[..., 256:] = top
+    c.q_pe.zero_()
+    got, lse = run(c)
+    want, want_lse = oracle_reference(c)
+    assert O.rel_l2(got, want) < 4e-3 and np.abs(lse - want_lse).max() <= 1e-3
