@@ -30,6 +30,9 @@
 // Warp roles (896 threads): 0-7 softmax + query load + epilogue, 8-23 dequantise (warp = 32 rows of a 64-channel panel), 24
 // QK^T issue, 25 L2 prefetch, 26 PV issue. Every wait is bounded (ptx::mbar_wait).
 #pragma once
+#include <climits>
+#include <type_traits>
+
 #include "mla_decode_sm100.cuh"
 
 namespace mla {
@@ -130,7 +133,9 @@ __device__ __forceinline__ void h16_prefetch_role(H16Smem& s, const DecodeParams
 // panel row (16 packed bytes = two scale blocks) of rows lane / 2 and 16 + lane / 2, so that a warp's load touches 16 lines
 // and its 16-byte stores are conflict-free. The warps of part A also move the rope panel (8 rows each, eight lanes per row).
 // The cache row of a token is looked up by one lane and handed round by shuffle. Rows past the request's end and rows of a
-// bad page id are never loaded: zero bytes, zero scale. The loads of tile t + 1 are issued as soon as tile t's bytes have
+// bad page id are never loaded: zero bytes, zero scale. With several query tokens per request the last tokens are not seen by
+// every row, and a row that masks a token multiplies its value with probability 0, so a NaN block scale must not reach that value:
+// there the block becomes 0, and the token's rope part, which only enters scores, NaN. The loads of tile t + 1 are issued as soon as tile t's bytes have
 // been converted, the page ids of tile t + 2 behind them.
 // ---------------------------------------------------------------------------------------------------------------
 template <bool part_a>  // whether the warp's panel belongs to part A
@@ -148,11 +153,13 @@ __device__ __forceinline__ void h16_convert_warps(H16Smem& s, const DecodeParams
   const uint8_t* const ckv0 = P.ckv + 32 * w + 16 * hh;
   const uint8_t* const sf0 = P.sf + 4 * w + 2 * hh;
   const uint8_t* const kpe0 = P.kpe + 8 * (lane & 7);
+  auto has_nan = [](uint32_t w) { return __vcmpeq4(w & 0x7F7F7F7Fu, 0x7F7F7F7Fu) != 0u; };
   for (int si = 0; si < n_segs; ++si) {
     const Seg seg = s.segs[si];
     const int nt = h16_tiles(seg);
     if (nt <= 0) continue;
     const int* pt = P.page_table + (long long)seg.b * P.pt_stride;
+    const int first_masked = P.q_len > 1 ? P.kv_lens[seg.b] - (P.q_len - 1) : INT_MAX;  // first token that some row does not see
     uint4 rw[2];
     uint32_t rs[2];
     uint2 rr[2];
@@ -183,12 +190,17 @@ __device__ __forceinline__ void h16_convert_warps(H16Smem& s, const DecodeParams
       }
       tok += kH16Tile;
     };
-    fetch_rows(fetch_id(tok));
-    int page = fetch_id(tok);
-    for (int t = 0; t < nt; ++t, ++it) {
-      const uint32_t kb = it & 1, buf = kb * uint32_t(sizeof(s.kv[0]));
-      // this part of the buffer was released by the MMAs of tile it - 2
-      if (it >= 2 && !__all_sync(~0u, ptx::mbar_wait(&freed[kb], ((it >> 1) - 1) & 1, &s.abort_flag))) return;
+    // the tile in the registers, into buffer `buf`; MASKED: rows from `first` on hold tokens that some query row does not see
+    auto convert = [&](auto masked, uint32_t buf, int first) {
+      constexpr bool MASKED = decltype(masked)::value;
+      if constexpr (MASKED) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (16 * u + (lane >> 1) < first) continue;
+          if ((rs[u] & 0x7Fu) == 0x7Fu) rs[u] &= 0xFF00u;
+          if ((rs[u] & 0x7F00u) == 0x7F00u) rs[u] &= 0x00FFu;
+        }
+      }
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const uint32_t s2 = ru[u] < 0 ? 0u : ptx::e4m3x2_to_f16x2(uint16_t(rs[u]));  // scales of the unit's two blocks
@@ -205,11 +217,30 @@ __device__ __forceinline__ void h16_convert_warps(H16Smem& s, const DecodeParams
       if constexpr (part_a) {
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-          const uint2 x = rj[j] < 0 ? make_uint2(0, 0) : rr[j];
+          uint2 x = rj[j] < 0 ? make_uint2(0, 0) : rr[j];
+          if constexpr (MASKED) {
+            if (rj[j] >= 0 && rope_row + 4 * j >= first) {
+              const uint4* sf = reinterpret_cast<const uint4*>(P.sf + (long long)rj[j] * 32);
+              const uint4 a = sf[0], b = sf[1];
+              if (has_nan(a.x) || has_nan(a.y) || has_nan(a.z) || has_nan(a.w) || has_nan(b.x) || has_nan(b.y) || has_nan(b.z) || has_nan(b.w))
+                x = make_uint2(0x7F7F7F7Fu, 0x7F7F7F7Fu);
+            }
+          }
           ptx::sts128(rope0 + buf + j * 512 + ((rope_c ^ (rope_s + 4 * j)) << 4), ptx::e4m3x2_to_f16x2(uint16_t(x.x)),
                       ptx::e4m3x2_to_f16x2(uint16_t(x.x >> 16)), ptx::e4m3x2_to_f16x2(uint16_t(x.y)), ptx::e4m3x2_to_f16x2(uint16_t(x.y >> 16)));
         }
       }
+    };
+    fetch_rows(fetch_id(tok));
+    int page = fetch_id(tok);
+    for (int t = 0; t < nt; ++t, ++it) {
+      const uint32_t kb = it & 1, buf = kb * uint32_t(sizeof(s.kv[0]));
+      // this part of the buffer was released by the MMAs of tile it - 2
+      if (it >= 2 && !__all_sync(~0u, ptx::mbar_wait(&freed[kb], ((it >> 1) - 1) & 1, &s.abort_flag))) return;
+      // a tile whose tokens every row sees (all but a request's last one, and that too with one query token) goes without the checks
+      const int tok0 = tok - kH16Tile - lane;  // token of this warp's first row
+      if (tok0 + 32 <= first_masked) convert(std::false_type(), buf, 0);
+      else convert(std::true_type(), buf, first_masked - tok0);
       ptx::fence_proxy_async_smem();
       __syncwarp();
       ptx::mbar_arrive_if(&full[kb], lane == 0);

@@ -159,3 +159,27 @@ def test_small_query_elements_against_large_latents(top):
     got, lse = run(c)
     want, want_lse = oracle_reference(c)
     assert O.rel_l2(got, want) < 4e-3 and np.abs(lse - want_lse).max() <= 1e-3
+
+
+@pytest.mark.parametrize("block", [0, 9, 17, 31])  # (both parts of the tile, in either CTA)
+def test_nan_scale_of_a_later_token_stays_out_of_earlier_query_tokens(block):
+    """A foreign cache may hold a NaN block scale. In one pass for all query tokens a row that must not see the token multiplies its
+    value with probability 0; the rows that do see it lose the partial result it is part of, as in a call of their own."""
+    lens, q_len, heads = [7, 65, 130, 64] * 60, 4, 16
+    c = SyntheticCache(lens, 64, heads, 0.5, 2.0, seed=3).to("cuda")
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q_nope = torch.randn(len(lens), q_len, heads, 512, generator=g, device="cuda").bfloat16()
+    q_pe = torch.randn(len(lens), q_len, heads, 64, generator=g, device="cuda").bfloat16()
+    args = (q_nope, q_pe, c.ckv_cache, c.ckv_sf_cache, c.kpe_cache, c.page_table, c.kv_lens, SM_SCALE, c.ckv_scale, c.kpe_scale)
+    assert _lib.load().nvfp4_mla_decode_multi_folds(len(lens), q_len, heads, 8192, 0) == 1
+    clean = serving.decode_multi_token(*args, max_kv_len=8192)
+    sf = c.ckv_sf_cache.view(torch.uint8)
+    for b, n in enumerate(lens):  # the last token of half of the requests, the last but two of the others
+        at = n - 1 if b % 8 < 4 else n - 3
+        sf[c.page_table[b, at // 64], at % 64, block] = 0x7F if b % 2 else 0xFF
+    out = serving.decode_multi_token(*args, max_kv_len=8192)
+    for b in range(len(lens)):
+        unaware = 3 if b % 8 < 4 else 1
+        assert torch.equal(out[b, :unaware], clean[b, :unaware]), b
+        if lens[b] <= 64:  # one partial result, lost
+            assert not out[b, unaware:].any()
