@@ -258,7 +258,9 @@ __device__ __forceinline__ void h16_convert_role(H16Smem& s, const DecodeParams&
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// roles: MMA issue
+// roles: MMA issue, by one elected thread behind a branch (an earlier form, every thread running the issue code with the MMAs
+// predicated on the elected one, gave wrong results where the warp happened to run it diverged, and was not faster: 64 heads, 32
+// ragged requests 147.5 us, this form 145.6)
 // ---------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void h16_qk_role(H16Smem& s, const DecodeParams& P, int n_segs, uint32_t& it, uint32_t& seg_count, int cg) {
   const bool leader = ptx::elect_one();
@@ -281,30 +283,32 @@ __device__ __forceinline__ void h16_qk_role(H16Smem& s, const DecodeParams& P, i
 #pragma unroll 1
           for (int p = 0; p < 4; ++p, q += 32, k += kH16Panel >> 4)
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks) ptx::mma_f16_ts_if(leader, tm + H16Cols::S, q + 8 * ks, k + 2 * ks, hi, idesc, ks ? 1u : accum | p);
+            for (int ks = 0; ks < 4; ++ks) ptx::mma_f16_ts_lo(tm + H16Cols::S, q + 8 * ks, k + 2 * ks, hi, idesc, ks ? 1u : accum | p);
         } else {
 #pragma unroll 1
           for (int p = 0; p < 4; ++p, q += kH16Rows * 128 >> 4, k += kH16Panel >> 4)
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks) ptx::mma_f16_ss_if(leader, tm + H16Cols::S, q + 2 * ks, k + 2 * ks, hi, idesc, ks ? 1u : accum | p);
+            for (int ks = 0; ks < 4; ++ks) ptx::mma_f16_ss_lo(tm + H16Cols::S, q + 2 * ks, k + 2 * ks, hi, idesc, ks ? 1u : accum | p);
         }
       };
       // the softmax warps have read the scores of tile it - 1; part A of this tile is in place
       if (!__all_sync(~0u, it < 1 || ptx::mbar_wait(&s.s_free, (it - 1) & 1, &s.abort_flag))) return;
       if (!__all_sync(~0u, ptx::mbar_wait(&s.full_a[kb], (it >> 1) & 1, &s.abort_flag))) return;
-      __syncwarp();  // (the issue code's operands live in uniform registers: the warp has to run it as one)
       ptx::tc_fence_after_sync();
-      half(cg ^ 1, 0u);
+      if (leader) {
+        half(cg ^ 1, 0u);
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-        ptx::mma_f16_ts_if(leader, tm + H16Cols::S, tm + H16Cols::QR + 8 * ks, k_lo + ((8 * kH16Panel + ks * 32) >> 4), hi, idesc, 1u);
-      if (leader) ptx::mma_commit(&s.free_a[kb]);
+        for (int ks = 0; ks < 4; ++ks)
+          ptx::mma_f16_ts_lo(tm + H16Cols::S, tm + H16Cols::QR + 8 * ks, k_lo + ((8 * kH16Panel + ks * 32) >> 4), hi, idesc, 1u);
+        ptx::mma_commit(&s.free_a[kb]);
+      }
       __syncwarp();
       if (!__all_sync(~0u, ptx::mbar_wait(&s.full_b[kb], (it >> 1) & 1, &s.abort_flag))) return;
-      __syncwarp();
       ptx::tc_fence_after_sync();
-      half(cg, 1u);
-      if (leader) ptx::mma_commit(&s.s_full);
+      if (leader) {
+        half(cg, 1u);
+        ptx::mma_commit(&s.s_full);
+      }
       __syncwarp();
     }
   }
@@ -320,13 +324,12 @@ __device__ __forceinline__ void h16_pv_role(H16Smem& s, const DecodeParams& P, i
     for (int t = 0; t < nt; ++t, ++it) {
       const uint32_t kb = it & 1;
       if (!__all_sync(~0u, ptx::mbar_wait(&s.p_full, it & 1, &s.abort_flag))) return;
-      __syncwarp();
       ptx::tc_fence_after_sync();
       const uint64_t v_desc = ptx::smem_desc_sw128(ptx::smem_u32(s.kv[kb][4 * cg]), kH16Panel, 1024);
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-        ptx::mma_f16_ts_if(leader, tm + H16Cols::O, tm + H16Cols::P + 8 * ks, uint32_t(v_desc) + ((ks * 16 * 128) >> 4), uint32_t(v_desc >> 32), idesc, (t | ks) != 0);
       if (leader) {
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          ptx::mma_f16_ts_lo(tm + H16Cols::O, tm + H16Cols::P + 8 * ks, uint32_t(v_desc) + ((ks * 16 * 128) >> 4), uint32_t(v_desc >> 32), idesc, (t | ks) != 0);
         ptx::mma_commit(&s.pv_done);
         ptx::mma_commit(&s.free_b[kb]);
       }

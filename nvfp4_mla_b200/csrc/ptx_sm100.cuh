@@ -323,26 +323,20 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accum)
       : "memory");
 }
-// The same two, issued by the one thread of the warp whose `lead` is set, without a branch, and with the operand descriptors
-// as their low words (start address and LBO; a K step or panel is one 32-bit addition) plus a constant high word: fewer
-// registers and instructions per MMA where a warp issues dozens of short ones per tile. The warp has to run them converged (a
-// __syncwarp in front): the operands live in uniform registers, which two diverged halves of a warp would share.
-__device__ __forceinline__ void mma_f16_ss_if(uint32_t lead, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc,
-                                              uint32_t accum) {
+// The same two with the operand descriptors as their low words (start address and LBO; a K step or panel is one 32-bit
+// addition) plus a constant high word: fewer registers and instructions per MMA where a thread issues dozens of short ones per tile.
+__device__ __forceinline__ void mma_f16_ss_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accum) {
   asm volatile(
-      "{\n.reg .pred p, q;\n.reg .b64 da, db;\nsetp.ne.b32 p, %5, 0;\nsetp.ne.b32 q, %6, 0;\n"
-      "mov.b64 da, {%1, %3};\nmov.b64 db, {%2, %3};\n"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accum), "r"(lead)
+      "{\n.reg .pred p;\n.reg .b64 da, db;\nsetp.ne.b32 p, %5, 0;\nmov.b64 da, {%1, %3};\nmov.b64 db, {%2, %3};\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accum)
       : "memory");
 }
-__device__ __forceinline__ void mma_f16_ts_if(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc,
-                                              uint32_t accum) {
+__device__ __forceinline__ void mma_f16_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accum) {
   asm volatile(
-      "{\n.reg .pred p, q;\n.reg .b64 db;\nsetp.ne.b32 p, %5, 0;\nsetp.ne.b32 q, %6, 0;\n"
-      "mov.b64 db, {%2, %3};\n"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accum), "r"(lead)
+      "{\n.reg .pred p;\n.reg .b64 db;\nsetp.ne.b32 p, %5, 0;\nmov.b64 db, {%2, %3};\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accum)
       : "memory");
 }
 __device__ __forceinline__ void mma_f8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accum) {

@@ -183,3 +183,28 @@ def test_nan_scale_of_a_later_token_stays_out_of_earlier_query_tokens(block):
         assert torch.equal(out[b, :unaware], clean[b, :unaware]), b
         if lens[b] <= 64:  # one partial result, lost
             assert not out[b, unaware:].any()
+
+
+@pytest.mark.parametrize("heads,q_len", [(64, 1), (128, 1), (16, 4), (144, 1)])
+def test_repeated_runs_give_the_same_bits(heads, q_len):
+    """A race between the kernel's roles, or an issue warp that loses its operands, shows as results that come and go: many ragged requests
+    (lengths from one token to fifty tiles), other batches in between, and every run equals the first bit for bit."""
+    rng = np.random.default_rng(heads)
+    lens = [int(x) for x in np.exp(rng.uniform(0, np.log(3200), 200))]
+    c = SyntheticCache(lens, 16, heads, 0.5, 2.0, seed=heads, device="cuda")
+    shape = (len(lens), q_len, heads)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q_nope, q_pe = torch.randn(*shape, 512, generator=g, device="cuda").bfloat16(), torch.randn(*shape, 64, generator=g, device="cuda").bfloat16()
+    call = serving.decode_multi_token
+    if q_len == 1:
+        call, q_nope, q_pe = mla.decode, q_nope[:, 0], q_pe[:, 0]
+
+    def once(n):
+        return call(q_nope[:n], q_pe[:n], c.ckv_cache, c.ckv_sf_cache, c.kpe_cache, c.page_table[:n], c.kv_lens[:n], SM_SCALE, c.ckv_scale,
+                    c.kpe_scale, max_kv_len=max(lens))
+
+    first = {n: once(n) for n in (200, 173)}
+    for i in range(60):
+        for n, want in first.items():
+            assert torch.equal(once(n), want), (i, n)
+    assert mla.workspace_status() == 0
