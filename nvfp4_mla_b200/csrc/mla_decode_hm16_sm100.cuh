@@ -537,17 +537,29 @@ __device__ __forceinline__ void h16_softmax_role(H16Smem& s, const DecodeParams&
     const float lt = s.xl[0][h] + s.xl[1][h];
     const float inv = lt > 0.f ? P.ckv_scale / lt : 0.f;
     const long long slot = (long long)seg.cta + seg.w;
-    float* orow = P.o_part + (slot * P.heads_per_cta + h) * CKV + 256 * cg + 128 * half;
+    // A thread holds a row, but a store of a row per lane touches 32 lines: 32 channels at a time turn through this warp's share of
+    // the quadrant's rows of s.q (the query is not needed any more), so that a store writes four rows' 128 bytes. The epilogue of
+    // a CTA with one segment of 128 rows took 12000 cycles with a row per lane and takes 8000; 64 heads, 32 ragged requests: 147.5 us
+    // before, 144.7 now; 128 heads, 64 requests of 300 tokens: 57.3, 54.7.
+    float* const orow = P.o_part + (slot * P.heads_per_cta + 32 * quad + (lane >> 3)) * CKV + 256 * cg + 128 * half + 4 * (lane & 7);
 #pragma unroll 1
     for (int c0 = 0; c0 < 128; c0 += 32) {
+      const uint32_t stage = ptx::smem_u32(s.q[2 * half + ((c0 >> 5) & 1)]) + 32 * quad * 128;
       uint32_t o[32];
       ptx::tmem_ld32(tm_lane + H16Cols::O + 128 * half + c0, o);
       ptx::tmem_wait_ld();
-      if (h < live_rows) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(orow + c0 + j) = make_float4(__uint_as_float(o[j]) * inv, __uint_as_float(o[j + 1]) * inv,
-                                                                  __uint_as_float(o[j + 2]) * inv, __uint_as_float(o[j + 3]) * inv);
+      for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * inv);
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        ptx::sts128(stage + lane * 128 + (uint32_t(c ^ (lane & 7)) << 4), o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {  // rows 4 i + lane / 8
+        const int r = 4 * i + (lane >> 3);
+        const uint4 w = ptx::lds128(stage + r * 128 + (uint32_t((lane ^ r) & 7) << 4));
+        if (32 * quad + r < live_rows)
+          *reinterpret_cast<float4*>(orow + 4 * i * CKV + c0) = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
       }
     }
     if (cg == 0 && half == 0 && h < live_rows) P.lse_part[slot * P.heads_per_cta + h] = lt > 0.f ? m + log2f(lt) : -INFINITY;
