@@ -41,7 +41,8 @@ NVFP4_MLA_API const char* nvfp4_mla_last_error(void);
 NVFP4_MLA_API int nvfp4_mla_decode_launches(int batch, int heads, int max_kv_len, int num_splits, int precision);
 
 /* Bytes of scratch nvfp4_mla_decode needs for this problem on the current device. `num_splits` as in the decode
- * call. Replaces the torch::empty of o_part / lse_part inside the reference launcher
+ * call. At 64 and more heads the size covers two groupings of the heads, of which the call uses one (128 heads, 64
+ * requests: 36 MB). Replaces the torch::empty of o_part / lse_part inside the reference launcher
  * (nvfp4_mla/csrc/mla_decode.cu:1042-1047). Returns -1 on invalid arguments. */
 NVFP4_MLA_API int64_t nvfp4_mla_decode_workspace_bytes(int batch, int heads, int num_splits);
 
@@ -103,7 +104,8 @@ NVFP4_MLA_API int nvfp4_mla_decode_multi(const void* q_nope, const void* q_pe, c
  *     batch * (heads / 16) * max(num_splits, 1) up to about 138 in either precision, e.g. batch 64 with 16 heads, or
  *     batch 16 with 128 heads. The 8-bit mode normally groups 32 or 128 heads per CTA, which needs more scratch than
  *     that; this entry point uses the widest grouping that fits and falls back to 16 heads per CTA (same results
- *     within the mode's tolerance, slower at 128 heads).
+ *     within the mode's tolerance, slower at 128 heads). The 16-bit mode's form for 64 and more heads never fits: such
+ *     calls run 16 heads per CTA here and take up to twice as long as through nvfp4_mla_decode.
  *   - Nothing is allocated or freed here, by CUDA or by any library, on any call.
  *   - The first call on each device looks up the array's device address (cudaGetSymbolAddress) and does the one-time
  *     kernel set-up; make that first call outside any stream capture.

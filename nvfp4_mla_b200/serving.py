@@ -58,8 +58,8 @@ class PagedLatentCache:
 
     Pages are handed out on the host (a free list), the page table and lengths live on the device, and every append
     goes through the CUDA cache writer. What a call has to tell the device (page ids, lengths, token positions) is put
-    together on the host, which knows all of it, and crosses in one copy from pinned memory: no call waits for the GPU. ``max_pages_per_request`` fixes the page-table width, ``max_kv_len`` the decode
-    launch shape, so a decode step can be captured in a CUDA graph once the pages of the step have been reserved.
+    together on the host, which knows all of it, and crosses in one copy from pinned memory: no call waits for the GPU's work (the first copies of a
+    size allocate pinned memory, which may). ``max_pages_per_request`` fixes the page-table width, ``max_kv_len`` the decode launch shape, so a decode step can be captured in a CUDA graph once the pages of the step have been reserved.
     """
 
     def __init__(self, num_pages, page_size, max_requests, max_pages_per_request, ckv_scale, kpe_scale, device="cuda"):
