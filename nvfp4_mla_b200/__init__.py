@@ -321,15 +321,20 @@ def quantize_append_paged_mla_kv_cache(ckv, kpe, batch_indices, positions, ckv_c
     ``kv_last_page_len`` is accepted and not needed. ``check=True`` synchronises and raises if a token pointed
     outside the tables (such tokens are skipped)."""
     nnz = _check_append(ckv, kpe, batch_indices, positions, ckv_cache, ckv_sf_cache, kpe_cache, kv_indices, kv_indptr)
+    status = torch.zeros(1, dtype=torch.int32, device=ckv_cache.device) if check else None
+    _append(nnz, ckv, kpe, batch_indices, positions, ckv_cache, ckv_sf_cache, kpe_cache, kv_indices, kv_indptr, ckv_scale, kpe_scale, status)
+    if check and int(status.item()) != 0:
+        raise RuntimeError("quantize_append: a token named a request, position or page outside the tables")
+
+
+def _append(nnz, ckv, kpe, batch_indices, positions, ckv_cache, ckv_sf_cache, kpe_cache, kv_indices, kv_indptr, ckv_scale, kpe_scale, status=None):
+    """The cache writer, its arguments checked."""
     P, ps = ckv_cache.shape[:2]
     dev = ckv_cache.device
-    status = torch.zeros(1, dtype=torch.int32, device=dev) if check else None
     _on_device(dev, lambda: _lib.check(_lib.load().nvfp4_mla_quantize_append(
         _ptr(ckv), _ptr(kpe), _ptr(batch_indices), _ptr(positions), nnz, _ptr(ckv_cache), _ptr(ckv_sf_cache),
         _ptr(kpe_cache), P, ps, _ptr(kv_indices), _ptr(kv_indptr), kv_indptr.numel() - 1, float(ckv_scale),
-        float(kpe_scale), _ptr(status) if check else None, torch.cuda.current_stream(dev).cuda_stream)))
-    if check and int(status.item()) != 0:
-        raise RuntimeError("quantize_append: a token named a request, position or page outside the tables")
+        float(kpe_scale), _ptr(status), torch.cuda.current_stream(dev).cuda_stream)))
 
 
 def workspace_status(device=None, clear=False):

@@ -11,7 +11,7 @@ import operator
 import numpy as np
 import torch
 
-from . import _PRECISIONS, CKV, KPE, _check_append, _decode, _lib, decode, quantize_append_paged_mla_kv_cache
+from . import _PRECISIONS, CKV, KPE, _append, _check_append, _decode, _lib, decode
 
 
 def decode_multi_token(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_table, kv_lens, sm_scale,
@@ -96,34 +96,37 @@ class PagedLatentCache:
         named more than once: its shares follow each other. Whatever refuses the call does so before the pool changes."""
         if not requests:
             raise IndexError("append needs at least one request")
-        width, known = self.page_table.shape[1], len(self._lens)
+        width, known, free, n_free, page_size = self.page_table.shape[1], len(self._lens), self._free, len(self._free), self.page_size
         slots, values = [], []  # entries of the page table and of the lengths, and what they become
         reqs, counts, ends = [], [], []  # per entry of the call: request, tokens, the request's length after it
-        grown, taken = {}, 0  # per request: [length, new pages]; pages taken from the end of the free list
+        grown, taken = {}, 0  # per request: [length, pages, new pages]; pages taken from the end of the free list
         for r, n in requests:
-            r, n = range(known)[r], operator.index(n)  # (a negative id counts from the end)
-            if n < 0:
-                raise ValueError("counts must not be negative")
-            to = grown.setdefault(r, [self._lens[r], []])
-            held = len(self._pages[r]) + len(to[1])
-            need = -(-(to[0] + n) // self.page_size) - held
-            if need > len(self._free) - taken or held + need > width:
-                raise RuntimeError("out of cache pages")
+            if type(r) is not int or type(n) is not int or r < 0 or r >= known or n < 0:
+                r, n = range(known)[r], operator.index(n)  # (a negative id counts from the end)
+                if n < 0:
+                    raise ValueError("counts must not be negative")
+            to = grown.get(r)
+            if to is None:
+                to = grown[r] = [self._lens[r], len(self._pages[r]), []]
+            end, held, fresh = to
+            to[0] = end = end + n
+            need = -(-end // page_size) - held
             if need > 0:
+                if taken + need > n_free or held + need > width:
+                    raise RuntimeError("out of cache pages")
                 at = r * width + held
                 slots += range(at, at + need)
-                fresh = self._free[-taken - 1:-taken - need - 1:-1]
-                values += fresh
-                to[1] += fresh
+                got = free[-taken - 1:-taken - need - 1:-1]
+                values += got
+                fresh += got
+                to[1] = held + need
                 taken += need
-            to[0] += n
             reqs.append(r)
             counts.append(n)
-            ends.append(to[0])
+            ends.append(end)
         slots += [known * width + r for r in grown]
-        values += [end for end, _ in grown.values()]
-        counts = np.array(counts)
-        nnz, n_slots = int(counts.sum()), len(slots)
+        values += [to[0] for to in grown.values()]
+        nnz, n_slots, counts, ends = sum(counts), len(slots), np.array(counts), np.array(ends)
         # position of token j of entry i: ends[i] - counts[i] + j
         first = np.cumsum(counts) - counts
 
@@ -138,12 +141,12 @@ class PagedLatentCache:
         words = told[8 * n_slots:].view(torch.int32)
         write = (ckv, kpe, words[n_slots:n_slots + nnz], words[n_slots + nnz:], self.ckv_cache, self.ckv_sf_cache, self.kpe_cache,
                  self.page_table.view(-1), self._kv_indptr)
-        if _check_append(*write) and (ckv.data_ptr() % 16 or kpe.data_ptr() % 4):
+        if _check_append(*write) and (ckv.data_ptr() % 16 or kpe.data_ptr() % 4):  # (the C entry would refuse that too late)
             raise RuntimeError("ckv must be 16-byte and kpe 4-byte aligned")
         self._tables.index_copy_(0, told[:8 * n_slots].view(torch.int64), words[:n_slots])
-        quantize_append_paged_mla_kv_cache(*write, None, self.ckv_scale, self.kpe_scale)
-        del self._free[len(self._free) - taken:]
-        for r, (end, fresh) in grown.items():
+        _append(nnz, *write, self.ckv_scale, self.kpe_scale)
+        del free[n_free - taken:]
+        for r, (end, _, fresh) in grown.items():
             self._lens[r] = end
             self._pages[r] += fresh
 
@@ -164,9 +167,11 @@ class PagedLatentCache:
         if torch.is_tensor(requests):
             table, lens = self.page_table[requests.to(self.page_table.device)], self.kv_lens[requests.to(self.page_table.device)]
         else:
-            ids = torch.tensor(requests)
-            if ids.dim() == 1 and ids.numel() and ids.dtype in (torch.int64, torch.int32):
-                ids = ids.numpy().astype(np.int64)
+            plain = type(requests) is list and requests and all(type(r) is int for r in requests)  # (the usual form; 5 us less than a tensor)
+            ids = np.array(requests, dtype=np.int64) if plain else torch.tensor(requests)
+            if plain or (ids.dim() == 1 and ids.numel() and ids.dtype in (torch.int64, torch.int32)):
+                if not plain:
+                    ids = ids.numpy().astype(np.int64)
                 if not (-len(self._lens) <= ids.min() and ids.max() < len(self._lens)):
                     raise IndexError("request id out of range")
                 ids %= len(self._lens)
