@@ -76,6 +76,16 @@ NVFP4_MLA_API int nvfp4_mla_decode(const void* q_nope, const void* q_pe, const u
                      float ckv_scale, float kpe_scale, int max_kv_len, int num_splits, int precision, void* out,
                      float* out_f32, float* lse, void* workspace, int64_t workspace_bytes, void* stream);
 
+/* nvfp4_mla_decode for a caller whose max_kv_len is far above the lengths (the capacity of a pool), but who has an idea of the
+ * longest request: `expected_kv_len` (0: none) replaces max_kv_len where the library chooses between its kernels by cost. It
+ * changes the time of the call, never its result's validity: longer requests are served as well. (No counterpart in the
+ * reference.) */
+NVFP4_MLA_API int nvfp4_mla_decode_expecting(const void* q_nope, const void* q_pe, const uint8_t* ckv_cache, const uint8_t* ckv_sf_cache,
+                     const uint8_t* kpe_cache, int64_t num_pages, int page_size, const int32_t* page_table,
+                     int64_t page_table_stride, const int32_t* kv_lens, int batch, int heads, float sm_scale,
+                     float ckv_scale, float kpe_scale, int max_kv_len, int expected_kv_len, int num_splits, int precision, void* out,
+                     float* out_f32, float* lse, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* nvfp4_mla_decode for q_len query tokens per request (speculative / multi-token verification): q_nope [batch, q_len, heads,
  * 512] and q_pe [batch, q_len, heads, 64], out / out_f32 / lse likewise. The q_len tokens are the last ones of the request's
  * kv_lens; token i attends to the first kv_lens - (q_len - 1 - i) tokens. All rows of a request share one pass over its

@@ -72,8 +72,9 @@ def _on_device(dev, call):
 
 
 def _decode(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_table, kv_lens, sm_scale, ckv_scale, kpe_scale,
-            max_kv_len, num_splits, precision, want_out, want_partial, partial_into=None, q_len=1):
+            max_kv_len, num_splits, precision, want_out, want_partial, partial_into=None, q_len=1, expected_kv_len=0):
     # q_len > 1: dimension 1 of the queries holds the heads of q_len query tokens, token by token
+    # expected_kv_len: longest request as far as the caller knows (0: max_kv_len); only chooses between kernels
     _check_cache(ckv_cache, ckv_sf_cache, kpe_cache)
     if q_nope.dim() != 3 or q_nope.shape[2] != CKV:
         raise RuntimeError("q_nope must be [batch, heads, 512]")
@@ -113,11 +114,15 @@ def _decode(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, page_table, kv_len
         stream = torch.cuda.current_stream(dev).cuda_stream
         ws = _workspace(dev, stream, _workspace_bytes(dev.index, B, H, int(num_splits)))
         out = torch.empty(B, H, CKV, dtype=torch.bfloat16, device=dev) if want_out else None
-        fn, rows = (lib.nvfp4_mla_decode, (H,)) if q_len == 1 else (lib.nvfp4_mla_decode_multi, (q_len, H // q_len))
+        fn, rows, bound = lib.nvfp4_mla_decode, (H,), (int(max_kv_len),)
+        if q_len > 1:
+            fn, rows = lib.nvfp4_mla_decode_multi, (q_len, H // q_len)
+        elif expected_kv_len:
+            fn, bound = lib.nvfp4_mla_decode_expecting, (int(max_kv_len), int(expected_kv_len))
         _lib.check(fn(
             q_nope.data_ptr(), q_pe.data_ptr(), ckv_cache.data_ptr(), ckv_sf_cache.data_ptr(), kpe_cache.data_ptr(), ckv_cache.shape[0], ps,
             page_table.data_ptr(), page_table.stride(0), kv_lens.data_ptr(), B, *rows, float(sm_scale), float(ckv_scale),
-            float(kpe_scale), int(max_kv_len), int(num_splits), int(precision), _ptr(out), _ptr(o32), _ptr(lse),
+            float(kpe_scale), *bound, int(num_splits), int(precision), _ptr(out), _ptr(o32), _ptr(lse),
             ws.data_ptr(), ws.numel(), stream))
         return out, o32, lse
 

@@ -18,6 +18,8 @@ SIGNATURES = {
     "nvfp4_mla_decode_launches": (_i32, [_i32, _i32, _i32, _i32, _i32]),
     "nvfp4_mla_decode": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _i64, _vp, _i32, _i32, _f32, _f32, _f32,
                                 _i32, _i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp]),
+    "nvfp4_mla_decode_expecting": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _i64, _vp, _i32, _i32, _f32, _f32, _f32,
+                                          _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp]),
     "nvfp4_mla_decode_multi_folds": (_i32, [_i32, _i32, _i32, _i32, _i32]),
     "nvfp4_mla_decode_multi": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp, _i64, _vp, _i32, _i32, _i32, _f32, _f32, _f32,
                                       _i32, _i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp]),

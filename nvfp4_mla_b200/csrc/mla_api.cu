@@ -300,12 +300,13 @@ int64_t nvfp4_mla_decode_workspace_bytes(int batch, int heads, int num_splits) {
   return a < 0 || b < 0 ? -1 : (a > b ? a : b);
 }
 
-// The decode call proper; `heads` counts the rows of all q_len query tokens of a request, `hpc_limit` caps the heads per CTA (see heads_per_cta).
+// The decode call proper; `heads` counts the rows of all q_len query tokens of a request, `hpc_limit` caps the heads per CTA
+// (see heads_per_cta), which are chosen for requests of `expected_kv_len` tokens (0: of the bound max_kv_len).
 static int decode_impl(const void* q_nope, const void* q_pe, const uint8_t* ckv_cache, const uint8_t* ckv_sf_cache,
                        const uint8_t* kpe_cache, int64_t num_pages, int page_size, const int32_t* page_table,
                        int64_t page_table_stride, const int32_t* kv_lens, int batch, int heads, float sm_scale, float ckv_scale,
                        float kpe_scale, int max_kv_len, int num_splits, int precision, void* out, float* out_f32, float* lse,
-                       void* workspace, int64_t workspace_bytes, void* stream, int hpc_limit, int q_len = 1) {
+                       void* workspace, int64_t workspace_bytes, void* stream, int hpc_limit, int q_len = 1, int expected_kv_len = 0) {
   g_error[0] = 0;
   MLA_CHECK(precision == NVFP4_MLA_PRECISION_BF16 || precision == NVFP4_MLA_PRECISION_FP8,
             "precision must be 0 (bf16) or 1 (fp8), got %d", precision);
@@ -321,7 +322,7 @@ static int decode_impl(const void* q_nope, const void* q_pe, const uint8_t* ckv_
   DeviceInfo* d;
   if (device_info(&d)) return 1;
   mla::Problem pb;
-  const int hpc = heads_per_cta(heads, precision, *d, hpc_limit, batch, max_kv_len);
+  const int hpc = heads_per_cta(heads, precision, *d, hpc_limit, batch, expected_kv_len > 0 ? expected_kv_len : max_kv_len);
   if (problem_of(batch, heads, max_kv_len, num_splits, schedule_units(*d, precision, hpc), hpc, &pb)) return 1;
   if (batch == 0) return 0;
   const mla::WsLayout L = mla::ws_layout(pb.n_cta, pb.items(), pb.heads_per_cta);
@@ -396,6 +397,16 @@ int nvfp4_mla_decode(const void* q_nope, const void* q_pe, const uint8_t* ckv_ca
   return decode_impl(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, num_pages, page_size, page_table, page_table_stride, kv_lens,
                      batch, heads, sm_scale, ckv_scale, kpe_scale, max_kv_len, num_splits, precision, out, out_f32, lse, workspace,
                      workspace_bytes, stream, 128);
+}
+
+int nvfp4_mla_decode_expecting(const void* q_nope, const void* q_pe, const uint8_t* ckv_cache, const uint8_t* ckv_sf_cache,
+                               const uint8_t* kpe_cache, int64_t num_pages, int page_size, const int32_t* page_table,
+                               int64_t page_table_stride, const int32_t* kv_lens, int batch, int heads, float sm_scale, float ckv_scale,
+                               float kpe_scale, int max_kv_len, int expected_kv_len, int num_splits, int precision, void* out, float* out_f32,
+                               float* lse, void* workspace, int64_t workspace_bytes, void* stream) {
+  return decode_impl(q_nope, q_pe, ckv_cache, ckv_sf_cache, kpe_cache, num_pages, page_size, page_table, page_table_stride, kv_lens,
+                     batch, heads, sm_scale, ckv_scale, kpe_scale, max_kv_len, num_splits, precision, out, out_f32, lse, workspace,
+                     workspace_bytes, stream, 128, 1, expected_kv_len);
 }
 
 int nvfp4_mla_decode_multi_folds(int batch, int q_len, int heads, int max_kv_len, int precision) {

@@ -164,6 +164,9 @@ class PagedLatentCache:
         ``q_pe [len(requests), heads, 64]``. Returns the latent output ``[n, heads, 512]``, or, with
         ``w_uv [heads, 512, v_head_dim]``, the value-space output ``[n, heads, v_head_dim]`` (the absorbed W_UV applied
         after attention)."""
+        if precision not in _PRECISIONS:
+            raise ValueError(f"precision must be one of {list(_PRECISIONS)}, got {precision!r}")
+        longest = 0  # (the bound is the pool's capacity: by itself it would choose the kernel for long requests)
         if torch.is_tensor(requests):
             table, lens = self.page_table[requests.to(self.page_table.device)], self.kv_lens[requests.to(self.page_table.device)]
         else:
@@ -175,11 +178,12 @@ class PagedLatentCache:
                 if not (-len(self._lens) <= ids.min() and ids.max() < len(self._lens)):
                     raise IndexError("request id out of range")
                 ids %= len(self._lens)
+                longest = max(1, max(self._lens[r] for r in ids.tolist()))
                 idx = self._to_device(ids.nbytes, lambda host: host.__setitem__(slice(None), ids.view(np.uint8))).view(torch.int64)
                 table, lens = self.page_table.index_select(0, idx), self.kv_lens.index_select(0, idx)
             else:  # a mask over all requests; what is neither ids nor a mask is refused by the indexing
                 idx = ids.to(self.page_table.device)
                 table, lens = self.page_table[idx].contiguous(), self.kv_lens[idx].contiguous()
-        out = decode(q_nope, q_pe, self.ckv_cache, self.ckv_sf_cache, self.kpe_cache, table, lens, sm_scale, self.ckv_scale,
-                     self.kpe_scale, max_kv_len=self.max_kv_len, precision=precision)
+        out = _decode(q_nope, q_pe, self.ckv_cache, self.ckv_sf_cache, self.kpe_cache, table, lens, sm_scale, self.ckv_scale, self.kpe_scale,
+                      self.max_kv_len, 0, _PRECISIONS[precision], True, False, expected_kv_len=longest)[0]
         return out if w_uv is None else torch.einsum("bhc,hcv->bhv", out, w_uv.to(out.dtype))

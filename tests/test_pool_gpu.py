@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import mla_oracle as O
+import nvfp4_mla_b200 as mla
 from nvfp4_mla_b200 import serving
 
 pytestmark = pytest.mark.gpu
@@ -132,3 +133,27 @@ def test_forms_of_request_ids():
     for ids in ([1.7], [1.0], [], np.array([1.0])):
         with pytest.raises(IndexError):
             pool.decode(ids, *q, 0.1)
+
+
+def test_decode_runs_the_kernel_of_the_lengths_and_not_of_the_capacity():
+    """A pool of long requests that holds short ones: the bits are those of a call whose bound is the longest request (the 16-head
+    kernel), not those of a call with the capacity as its bound. Lengths that a program advances on the device by itself are served
+    in full all the same (rel-L2 < 4e-3 between two kernels of the 16-bit mode, as in the other tests)."""
+    pool = serving.PagedLatentCache(40, 64, 8, 4096, 0.5, 2.0)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    r = lambda *shape: torch.randn(*shape, generator=g, device="cuda").bfloat16()
+    lens = [40, 300, 5, 130, 77, 200, 1, 290]
+    pool.append(list(enumerate(lens)), r(sum(lens), 512), r(sum(lens), 64))
+    q = r(8, 64, 512), r(8, 64, 64)
+
+    def decode(bound):
+        return mla.decode(*q, pool.ckv_cache, pool.ckv_sf_cache, pool.kpe_cache, pool.page_table, pool.kv_lens, 0.07, 0.5, 2.0, max_kv_len=bound)
+
+    got = pool.decode(list(range(8)), *q, 0.07)
+    assert torch.equal(got, decode(300)) and not torch.equal(got, decode(pool.max_kv_len))
+    pool.kv_lens += 300 * (pool.kv_lens == 300).int()  # (past the request's pages: page 0's rows, for both)
+    pool.kv_lens += 1
+    got, want = pool.decode(list(range(8)), *q, 0.07).float(), decode(pool.max_kv_len).float()
+    assert O.rel_l2(got.cpu().numpy(), want.cpu().numpy()) < 4e-3
+    with pytest.raises(ValueError, match="precision"):
+        pool.decode([0], q[0][:1], q[1][:1], 0.07, precision="fp4")
