@@ -69,7 +69,15 @@ constexpr int kRawSlotsHm = 4;  // heads-as-M kernel: staging slots of 32 tokens
 //   heads-as-M kernel : 42 + 3.6 per tile of the fullest pair + 8.4 per (request, head group) and pair
 // Measured (16-head / heads-as-M), heads, requests, tokens: 64,8,2560: 27 / 42; 128,2,16000: 50 / 56; 128,1,51200: 62 / 54;
 // 64,128,800: 118 / 97; 128,32,1000: 74 / 47; 128,128,625: 146 / 122; 64,32 ragged 500..16000: 172 / 136; 128,64,16384:
-// 833 / 420; 128,2,1M: 1740 / 881.
+// 833 / 420; 128,2,1M: 1740 / 881. (Since then a segment's epilogue costs the heads-as-M kernel 2 us less.)
+//
+// `max_kv_len` is the bound, or what the caller expects. A bound far above the lengths sends few short requests to the heads-as-M
+// kernel, which has the higher fixed cost: with a bound of 131072, 40 sizes of 64 and 128 heads, 1 to 32 requests of 300 to 16000
+// tokens (16-head / this): 24.6 / 30.7 for one short request of 128 heads, at worst 32.3 / 45.0 (64 heads, 8 of
+// 2500 tokens) and 35.2 / 47.1 (64 heads, 32 of 300). The other error costs more: 229 / 141 (128 heads, 16 of 16000), 1740 / 881. So
+// the bound decides for this kernel, and callers that know better say so (nvfp4_mla_decode_expecting). Letting the device choose by the
+// lengths was measured: roles of both kernels in one, +10 us on every call of it; both kernels launched, the second leaving at once,
+// +2 to 5 us on every call of this kernel and 30.7 instead of 24.6 on the short ones.
 constexpr int kHm16MinHeads = 64;
 bool wants_hm16(int heads, int batch, int max_kv_len, const DeviceInfo& d) {
   if (heads < kHm16MinHeads || batch <= 0 || max_kv_len <= 0) return false;

@@ -13,7 +13,7 @@
 // one fused multiply-add, anything else by the real division. The block scale and the rope pair are treated alike; a
 // power-of-two rope scale needs no enclosure, its products are exact.
 //
-// 1152 bytes in, 352 bytes out per token, bound by instruction issue (278 warp instructions per token, 69 % of the issue slots):
+// 1152 bytes in, 352 bytes out per token, bound by instruction issue (343 warp instructions per token, 73 % of the issue slots):
 // 596415 tokens in 219.6 us, 233.7 with the divisions of the block scale and the rope (138 at the measured copy bandwidth).
 // Thirty-two tokens per warp with one walk through the page tables for all of them was slower (246.7 us).
 // One warp per token per trip; lane l owns scale block l
