@@ -170,15 +170,18 @@ class PagedLatentCache:
         if torch.is_tensor(requests):
             table, lens = self.page_table[requests.to(self.page_table.device)], self.kv_lens[requests.to(self.page_table.device)]
         else:
-            plain = type(requests) is list and requests and all(type(r) is int for r in requests)  # (the usual form; 5 us less than a tensor)
-            ids = np.array(requests, dtype=np.int64) if plain else torch.tensor(requests)
-            if plain or (ids.dim() == 1 and ids.numel() and ids.dtype in (torch.int64, torch.int32)):
-                if not plain:
-                    ids = ids.numpy().astype(np.int64)
-                if not (-len(self._lens) <= ids.min() and ids.max() < len(self._lens)):
+            if type(requests) is list and requests and all(type(r) is int for r in requests):  # (the usual form, without a tensor)
+                ids = requests
+            else:
+                ids = torch.tensor(requests)
+                if ids.dim() == 1 and ids.numel() and ids.dtype in (torch.int64, torch.int32):
+                    ids = ids.tolist()
+            if type(ids) is list:
+                known = len(self._lens)
+                if not (-known <= min(ids) and max(ids) < known):
                     raise IndexError("request id out of range")
-                ids %= len(self._lens)
-                longest = max(1, max(self._lens[r] for r in ids.tolist()))
+                longest = max(1, max(self._lens[r] for r in ids))
+                ids = np.array([r % known for r in ids], dtype=np.int64)
                 idx = self._to_device(ids.nbytes, lambda host: host.__setitem__(slice(None), ids.view(np.uint8))).view(torch.int64)
                 table, lens = self.page_table.index_select(0, idx), self.kv_lens.index_select(0, idx)
             else:  # a mask over all requests; what is neither ids nor a mask is refused by the indexing
